@@ -24,12 +24,21 @@ int check_launch(const char* what);
 // y <- y * (1.5 - 0.5 * d * y * y), starting from the hardware estimate.
 // One step brings the MUFU estimate to about one ulp.  A non-positive or NaN
 // pivot yields NaN/Inf, which the factorization propagates.
+// NORMAL: the caller checks that d is a normal number (pivot_normal), for
+// which the flush-to-zero estimate gives rsqrtf's bits without its scaling of
+// subnormal ones (17 against 40 cycles of latency on B200, once per pivot).
+template <bool NORMAL = false>
 __device__ __forceinline__ float rsqrt_refined(float d) {
-  float y = rsqrtf(d);
+  float y;
+  if (NORMAL)
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  else
+    y = rsqrtf(d);
   float h = 0.5f * d;
   float t = fmaf(-h * y, y, 0.5f);  // 0.5 - 0.5*d*y^2
   return fmaf(y, t, y);             // y + y*(0.5 - 0.5*d*y^2)
 }
+__device__ __forceinline__ bool pivot_normal(float d) { return d >= 1.17549435e-38f; }
 
 __device__ __forceinline__ bool pivot_bad(float d) { return !(d > 0.0f); }
 

@@ -1,24 +1,34 @@
 // Factor (and invert) one 64x64 diagonal block with four warps.
 //
-// Factorization (diag64_factor): the block is split 2x2 into 32x32 pieces
-// and three warps run concurrently, handing columns to each other through
-// shared memory:
+// Right-looking over four panels of 16 columns.  The rows of a panel are dealt
+// to warps 16 at a time: lanes 16..31 of panel warp w hold one row each of the
+// w-th 16-row block below the diagonal block, and lanes 0..15 of every panel
+// warp hold the diagonal block's own rows.  So each warp factors the 16x16
+// diagonal block itself (redundantly) and solves its rows in the same
+// instructions, and no value crosses warps inside a panel.  Four pivots at a
+// time, the 4x4 diagonal piece is shuffled to every lane and every lane runs
+// its little factorization, so that the chain from one pivot to the next is a
+// reciprocal square root, a multiply and a fused multiply-add; solved columns
+// reach the rest of the panel by shuffles.
 //
-//   warp 0   rows 0..31:                 pivots 0..31 (look-ahead warp factor)
-//   warp 1   rows 32..63, columns < 32:  L21 = A21 L11^{-T}, column by column
-//            behind warp 0
-//   warp 2   rows 32..63, columns >= 32: A22 -= L21 L21^T column by column
-//            behind warp 1, then pivots 32..63
+// Between panels all four warps apply the finished panel to the next one
+// (rank 16, in register tiles).  The columns beyond it are warp 2's, beside
+// the next panel, since it runs out of panel rows first.  The inverse T =
+// L^{-1} (diag64_factor_invert) is formed beside the panels as well, one
+// column per lane, by the warps that have no panel rows (any more), block row
+// by block row as the panels appear: T11 and T22 by substitution, -W = -L21
+// T11 below T11, and at the end T21 = -T22 W by all four warps.
 //
-// so that L21 and the A22 update hide behind the pivot chain.  A producer
-// advances a progress counter (release store) after every group of
-// kDiagGroup published columns; a consumer polls it with plain volatile loads
-// once per group and fences after success.  Every poll is bounded.
+// Every element of L receives the multiply-adds of the textbook right-looking
+// update, one by one in its order, so L does not depend on the blocking.
 //
-// Inverse (diag64_factor_invert): after the factorization, T11 = L11^{-1}
-// and T22 = L22^{-1} (one column per lane, warps 0 and 1), then
-// W^T = T11^T L21^T and T21^T = -W^T T22^T (all four warps), written
-// straight into the transposed layout the panel multiply reads.
+// What bounds it: the chain of 64 pivots (about 65 cycles each), then the
+// three updates between panels (about 650 each).  Measured on B200, one CTA
+// per SM, cycles: factor 7.6k, with the inverse 11.3k, and up to 1k more when
+// its code is not in the instruction cache.  Before it (a pipeline of three
+// warps over 32-wide halves, fully unrolled, one trip to another lane per
+// pivot, and the inverse after the factor): 12.6k and 17.3k, and 18.9k and
+// 27.8k with cold code, which is how a kernel that runs it once meets it.
 //
 // Rows and columns at or beyond the block's true width are identity
 // padding, so a short last block (w < 64) runs the same code.
@@ -30,9 +40,6 @@ namespace b2p {
 
 constexpr int kD64Ld = 68;   // row stride of S, T and the L^T view (floats)
 constexpr int kD64Threads = 128;
-constexpr int kDiagTimeout = -2;   // returned when a bounded wait gave up
-constexpr int kDiagGroup = 4;      // columns per hand-off between warps
-constexpr uint32_t kProgPolls = 1u << 22;
 
 // Barrier used between the engine's phases: the whole CTA, or a named
 // barrier over the first N threads (when other warps of the CTA run a
@@ -66,193 +73,304 @@ struct Diag64Smem {
   float p21t[32 * kLtLd];
   float w21[32 * kLtLd];
   float invd[64];         // 1 / diag(L)
-  int bad[2];
-  int prog[4];            // columns published by warps 0, 1, 2
-  int err;                // a bounded wait gave up
+  int bad[4];             // first bad pivot within each panel, or -1
 };
 
 __device__ __forceinline__ float* diag64_lt(Diag64Smem& sm) { return sm.lt0; }
 __device__ __forceinline__ const float* diag64_lt(const Diag64Smem& sm) { return sm.lt0; }
 static_assert(4 * 32 * kLtLd >= 64 * kD64Ld, "the L^T view must fit lt0..w21");
 
-// ---- progress counters -------------------------------------------------------
-__device__ __forceinline__ void prog_store(int* p, int v) {
-  asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v) : "memory");
-}
-// Called by all lanes at every column k of a consumer loop: at the first
-// column of each group, wait (bounded) until the producer has published the
-// whole group (its counter exceeds min(k + kDiagGroup - 1, last)).
-__device__ __forceinline__ bool prog_wait_group(const int* p, int k, int last) {
-  if (k % kDiagGroup != 0) return true;
-  const int want = min(k + kDiagGroup - 1, last);
-  const volatile int* vp = p;
-  for (uint32_t i = 0; i < kProgPolls; ++i) {
-    if (*vp > want) {
-      __threadfence_block();
-      return true;
-    }
-  }
-  return false;
-}
-// Producer side: after column k (of `last`), publish the group if complete.
-__device__ __forceinline__ void prog_publish(int* p, int k, int last, int lane) {
-  if (k % kDiagGroup == kDiagGroup - 1 || k == last) {
-    __syncwarp();
-    if (lane == 0) prog_store(p, k + 1);
-  }
-}
-
-// One warp factors the 32x32 block x (row `lane`) with the look-ahead update
-// of warp_factor32, publishing column k into lt[k * kD64Ld + lane] (0 above
-// the diagonal) and 1/L[k][k] into invd[k]; *prog counts published columns.
-// Returns the first bad local pivot or -1.
-//
-// The rank-1 update of column k beyond column k+1 is deferred by one step:
-// step k first shuffles pivot k out, then applies column k-1 (read back from
-// its publication) to columns k+1.., which fills the latency of pivot k's
-// reciprocal square root, and only then updates column k+1 with column k
-// (the look-ahead) and publishes column k.  Every element receives the same
-// fused multiply-adds in the same order as with the update done at once.
-// On B200 this took the 64x64 factorization from 16.4k to 12.7k cycles.
-__device__ __forceinline__ int warp_factor32_publish(float (&x)[32], int lane, float* lt, float* invd, int* prog) {
-  int bad = -1;
-  float lprev = 0.0f;  // this lane's L[lane][k-1]
+// ---- 16-wide pieces: one row (or one right-hand side) per lane ---------------
+__device__ __forceinline__ void load_row16(float (&x)[16], const float* src) {
 #pragma unroll
-  for (int k = 0; k < 32; ++k) {
-    const float d = __shfl_sync(kFullMask, x[k], k);
-    const float e = (k + 1 < 32) ? __shfl_sync(kFullMask, x[k], k + 1) : 0.0f;
-    // Column k-1's update of columns k+1.. (column k had it by look-ahead).
-    if (k >= 1 && k + 1 < 32) {
-      const float* col = lt + (k - 1) * kD64Ld;
-#pragma unroll
-      for (int j4 = (k + 1) / 4; j4 < 8; ++j4) {
-        const float4 c = reinterpret_cast<const float4*>(col)[j4];
-        const float cv[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int j = 4 * j4 + q;
-          if (j > k) x[j] = fmaf(-lprev, cv[q], x[j]);
-        }
-      }
-    }
-    if (bad < 0 && pivot_bad(d)) bad = k;
-    const float y = rsqrt_refined(d);
-    const float l = (lane == k) ? d * y : x[k] * y;
-    x[k] = l;
-    if (k + 1 < 32) x[k + 1] = fmaf(-l, e * y, x[k + 1]);
-    lt[k * kD64Ld + lane] = (lane >= k) ? l : 0.0f;
-    if (lane == k) invd[k] = y;
-    lprev = l;
-    // The column is read back by every lane next step, and by warp 1 / 2.
-    __syncwarp();
-    prog_publish(prog, k, 31, lane);
-  }
-  return bad;
-}
-
-__device__ __forceinline__ void load_row32(float (&x)[32], const float* src) {
-#pragma unroll
-  for (int c4 = 0; c4 < 8; ++c4) {
+  for (int c4 = 0; c4 < 4; ++c4) {
     const float4 v = reinterpret_cast<const float4*>(src)[c4];
     x[4 * c4] = v.x, x[4 * c4 + 1] = v.y, x[4 * c4 + 2] = v.z, x[4 * c4 + 3] = v.w;
   }
 }
-// Row of 32 to shared memory, zeros right of column `diag` (all if diag >= 31).
-__device__ __forceinline__ void store_row32(float* dst, const float (&x)[32], int diag) {
+__device__ __forceinline__ void store_row16(float* dst, const float (&x)[16]) {
 #pragma unroll
-  for (int c4 = 0; c4 < 8; ++c4) {
-    float v[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = (4 * c4 + q <= diag) ? x[4 * c4 + q] : 0.0f;
-    reinterpret_cast<float4*>(dst)[c4] = make_float4(v[0], v[1], v[2], v[3]);
-  }
+  for (int c4 = 0; c4 < 4; ++c4)
+    reinterpret_cast<float4*>(dst)[c4] = make_float4(x[4 * c4], x[4 * c4 + 1], x[4 * c4 + 2], x[4 * c4 + 3]);
 }
 
-// Factor the block in sm.S (lower triangle and diagonal read; the caller has
-// filled it and synchronised).  On return sm.S holds L in its lower triangle
-// (the upper-right 32x32 block is left as it was), the L^T view holds
-// Lt[m][j] = L[j][m] for j >= m (other entries unspecified) and sm.invd
-// 1/diag(L).  Returns the first bad pivot, -1, or kDiagTimeout.  Every thread
-// of the CTA calls it; threads beyond the first three warps only take part
-// in the barriers.
-template <class Bar = CtaBarrier>
-__device__ __forceinline__ int diag64_factor(Diag64Smem& sm, Bar bar = Bar()) {
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int warp = tid >> 5;
-  float* Lt = diag64_lt(sm);
-  if (tid < 4) sm.prog[tid] = 0;
-  if (tid == 0) sm.err = 0;
-  bar();
-  if (warp == 0) {
-    float x[32];
-    load_row32(x, sm.S + lane * kD64Ld);
-    const int b = warp_factor32_publish(x, lane, Lt, sm.invd, &sm.prog[0]);
-    if (lane == 0) sm.bad[0] = b;
-    store_row32(sm.S + lane * kD64Ld, x, lane);
-  } else if (warp == 1) {
-    // L21 row 32 + lane.
-    float x[32];
-    load_row32(x, sm.S + (32 + lane) * kD64Ld);
-    bool ok = true;
+// The rank-16 update in register tiles of R rows by 4 columns, x[4r + c] -=
+// sum_m a_rm lt[m][c0 + c], m = 0..15 ascending.  The columns' factors come
+// from the L^T view, where a warp's reads of one m are contiguous; so do the
+// rows' (`lt_r`, a_rm = lt_r[m][r]) or, for T, they are rows of T^T (`tt`,
+// a_rm = tt[r][m]).
+template <int R, bool TROWS>
+__device__ __forceinline__ void update_tile16(float (&x)[4 * R], const float* rows, const float* lt_c) {
+#pragma unroll 2
+  for (int m = 0; m < 16; m += 4) {
+    float a[4][R];
+    if (TROWS) {
 #pragma unroll
-    for (int k = 0; k < 32; ++k) {
-      if (ok && !prog_wait_group(&sm.prog[0], k, 31)) ok = false;
-      const float l = x[k] * sm.invd[k];
-      x[k] = l;
-      Lt[k * kD64Ld + 32 + lane] = l;
-      prog_publish(&sm.prog[1], k, 31, lane);
-      if (k + 1 < 32) {
-        const float* col = Lt + k * kD64Ld;
+      for (int r = 0; r < R; ++r) {
+        const float4 v = *reinterpret_cast<const float4*>(rows + r * kD64Ld + m);
+        a[0][r] = v.x, a[1][r] = v.y, a[2][r] = v.z, a[3][r] = v.w;
+      }
+    } else {
 #pragma unroll
-        for (int j4 = (k + 1) / 4; j4 < 8; ++j4) {
-          const float4 c = reinterpret_cast<const float4*>(col)[j4];
-          const float cv[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int j = 4 * j4 + q;
-            if (j > k) x[j] = fmaf(-l, cv[q], x[j]);
-          }
+      for (int p = 0; p < 4; ++p) {
+        if (R == 4) {
+          const float4 v = *reinterpret_cast<const float4*>(rows + (m + p) * kD64Ld);
+          a[p][0] = v.x, a[p][1] = v.y, a[p][R - 2] = v.z, a[p][R - 1] = v.w;
+        } else {
+          const float2 v = *reinterpret_cast<const float2*>(rows + (m + p) * kD64Ld);
+          a[p][0] = v.x, a[p][1] = v.y;
         }
       }
     }
-    store_row32(sm.S + (32 + lane) * kD64Ld, x, 31);
-    if (!ok) sm.err = 1;
-  } else if (warp == 2) {
-    // A22 row 32 + lane (columns 32..63): update, then factor.
-    float x[32];
-    load_row32(x, sm.S + (32 + lane) * kD64Ld + 32);
-    bool ok = true;
-#pragma unroll 4
-    for (int k = 0; k < 32; ++k) {
-      if (ok && !prog_wait_group(&sm.prog[1], k, 31)) ok = false;
-      const float* col = Lt + k * kD64Ld + 32;
-      const float l = col[lane];
 #pragma unroll
-      for (int j4 = 0; j4 < 8; ++j4) {
-        const float4 c = reinterpret_cast<const float4*>(col)[j4];
-        x[4 * j4 + 0] = fmaf(-l, c.x, x[4 * j4 + 0]);
-        x[4 * j4 + 1] = fmaf(-l, c.y, x[4 * j4 + 1]);
-        x[4 * j4 + 2] = fmaf(-l, c.z, x[4 * j4 + 2]);
-        x[4 * j4 + 3] = fmaf(-l, c.w, x[4 * j4 + 3]);
+    for (int p = 0; p < 4; ++p) {
+      const float4 b = *reinterpret_cast<const float4*>(lt_c + (m + p) * kD64Ld);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        x[4 * r + 0] = fmaf(-a[p][r], b.x, x[4 * r + 0]);
+        x[4 * r + 1] = fmaf(-a[p][r], b.y, x[4 * r + 1]);
+        x[4 * r + 2] = fmaf(-a[p][r], b.z, x[4 * r + 2]);
+        x[4 * r + 3] = fmaf(-a[p][r], b.w, x[4 * r + 3]);
       }
     }
-    const int b = warp_factor32_publish(x, lane, Lt + 32 * kD64Ld + 32, sm.invd + 32, &sm.prog[2]);
-    if (lane == 0) sm.bad[1] = b;
-    store_row32(sm.S + (32 + lane) * kD64Ld + 32, x, lane);
-    if (!ok) sm.err = 1;
   }
-  bar();
-  if (sm.err) return kDiagTimeout;
-  const int b0 = sm.bad[0], b1 = sm.bad[1];
-  return b0 >= 0 ? b0 : (b1 >= 0 ? 32 + b1 : -1);
+}
+
+// The tile's R rows of four at `dst` (row stride kD64Ld), less panels
+// k0 .. k1 - 1 of L (`rows`, `lt_c` as above, at panel 0).
+template <int R, bool TROWS>
+__device__ __forceinline__ void update_blocks(float* dst, const float* rows, const float* lt_c, int k0, int k1) {
+  float x[4 * R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const float4 v = *reinterpret_cast<const float4*>(dst + r * kD64Ld);
+    x[4 * r] = v.x, x[4 * r + 1] = v.y, x[4 * r + 2] = v.z, x[4 * r + 3] = v.w;
+  }
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k)
+    update_tile16<R, TROWS>(x, rows + 16 * k * (TROWS ? 1 : kD64Ld), lt_c + 16 * k * kD64Ld);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    *reinterpret_cast<float4*>(dst + r * kD64Ld) = make_float4(x[4 * r], x[4 * r + 1], x[4 * r + 2], x[4 * r + 3]);
+}
+
+// x <- L^{-1} x for the 16x16 lower L at lt (lt[m * kD64Ld + j] = L[j][m]) and
+// invd, by right-looking forward substitution.
+__device__ __forceinline__ void subst16(float (&x)[16], const float* lt, const float* invd) {
+#pragma unroll
+  for (int m = 0; m < 16; ++m) {
+    x[m] *= invd[m];
+#pragma unroll
+    for (int j4 = (m + 1) / 4; j4 < 4; ++j4) {
+      const float4 c = reinterpret_cast<const float4*>(lt + m * kD64Ld)[j4];
+      const float cv[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = 4 * j4 + q;
+        if (j > m) x[j] = fmaf(-x[m], cv[q], x[j]);
+      }
+    }
+  }
+}
+
+// Factors the 16x16 block held by lanes 0..15 (row `lane`) and solves the
+// rows of lanes 16..31 against it; 1/L[k][k] goes to invd.  A group of four
+// columns updates the next four at once and the rest during the next group's
+// chain.  NORMAL (see rsqrt_refined): returns 0, or a non-zero value if a
+// pivot was not a normal positive number, and the caller starts again with
+// the general form; that returns the first bad local pivot or -1.  The answer
+// is the same on every lane.
+template <bool NORMAL>
+__device__ __forceinline__ int factor16(float (&x)[16], int lane, float* invd) {
+  int bad = NORMAL ? 0 : -1;
+  float lp[4] = {0.f, 0.f, 0.f, 0.f};  // this lane's L of the previous group
+#pragma unroll
+  for (int k = 0; k < 16; k += 4) {
+    float a[4][4], f[4][4], y[4], l[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int r = c; r < 4; ++r) a[r][c] = __shfl_sync(kFullMask, x[k + c], k + r);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      if (k >= 4) {
+#pragma unroll
+        for (int j = k + 4; j < 16; ++j) x[j] = fmaf(-lp[p], __shfl_sync(kFullMask, lp[p], j), x[j]);
+      }
+      const float d = a[p][p];
+      if (NORMAL)
+        bad |= pivot_normal(d) ? 0 : 1;
+      else if (bad < 0 && pivot_bad(d))
+        bad = k + p;
+      y[p] = rsqrt_refined<NORMAL>(d);
+#pragma unroll
+      for (int r = p + 1; r < 4; ++r) a[r][p] *= y[p];
+      l[p] = (lane == k + p) ? d * y[p] : x[k + p] * y[p];
+#pragma unroll
+      for (int c = p + 1; c < 4; ++c) {
+#pragma unroll
+        for (int r = c; r < 4; ++r) a[r][c] = fmaf(-a[r][p], a[c][p], a[r][c]);
+        x[k + c] = fmaf(-l[p], a[c][p], x[k + c]);
+      }
+      if (k < 12) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) f[r][p] = __shfl_sync(kFullMask, l[p], k + 4 + r);
+      }
+      x[k + p] = l[p];
+    }
+    if (k < 12) {
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) x[k + 4 + r] = fmaf(-l[p], f[r][p], x[k + 4 + r]);
+        lp[p] = l[p];
+      }
+    }
+    if (threadIdx.x == 0) *reinterpret_cast<float4*>(invd + k) = make_float4(y[0], y[1], y[2], y[3]);
+  }
+  return bad;
 }
 
 // diag64_factor's result as every thread of the CTA can read it back once
 // the factorization's last barrier has been passed by all of them.
 __device__ __forceinline__ int diag64_status(const Diag64Smem& sm) {
-  if (sm.err) return kDiagTimeout;
-  return sm.bad[0] >= 0 ? sm.bad[0] : (sm.bad[1] >= 0 ? 32 + sm.bad[1] : -1);
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+    if (sm.bad[p] >= 0) return 16 * p + sm.bad[p];
+  return -1;
+}
+
+// The engine's body, see the top of the file; INVERT adds T = L^{-1}.
+// Phase ph (0..3) factors panel ph; with INVERT a phase 4 ends the inverse.
+template <bool INVERT, class Bar>
+__device__ __forceinline__ int diag64_run(Diag64Smem& sm, Bar bar) {
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int warp = tid >> 5;
+  float* S = sm.S;
+  float* Lt = diag64_lt(sm);
+  float* TT = sm.T;
+#pragma unroll 1
+  for (int ph = 0; ph < (INVERT ? 5 : 4); ++ph) {
+    if (ph > 0 && ph < 4) {
+      // Panel ph - 1 applied to column block ph: rows 16 ph .. 63, two rows
+      // and four columns a thread.
+      const int r = 16 * ph + 2 * (tid >> 2), c = 16 * ph + 4 * (tid & 3);
+      if (r < 64) update_blocks<2, false>(S + r * kD64Ld + c, Lt + r, Lt + c, ph - 1, ph);
+      bar();
+    }
+    float x[16];
+    float* row = nullptr;
+    if (ph < 4 && warp < 3 && (warp + ph < 3 || warp == 0)) {
+      // The panel.  The last one has no rows for lanes 16..31.
+      const int r = 16 * (lane < 16 ? ph : ph + warp) + lane;
+      const bool live = r < 64;
+      row = S + (live ? r : 48) * kD64Ld + 16 * ph;
+      load_row16(x, row);
+      int b = factor16<true>(x, lane, sm.invd + 16 * ph);
+      if (b != 0) {
+        load_row16(x, row);
+        b = factor16<false>(x, lane, sm.invd + 16 * ph);
+      } else {
+        b = -1;
+      }
+      if (tid == 0) sm.bad[ph] = b;
+      // The diagonal block is warp 0's to write, zero above its diagonal; into
+      // S after the barrier, since every panel warp reads it there.
+      if (live && (lane >= 16 || warp == 0)) {
+        if (lane >= 16) store_row16(row, x);
+        if (lane < 16) {
+#pragma unroll
+          for (int c = 0; c < 16; ++c) x[c] = c <= lane ? x[c] : 0.0f;
+        }
+        float* lc = Lt + 16 * ph * kD64Ld + r;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) lc[c * kD64Ld] = x[c];
+      }
+    } else if ((warp == 2 && ph < 3) || (!INVERT && warp == 3 && ph == 1)) {
+      // Panels before ph applied to the columns beyond block ph: warp 2 one
+      // block ahead; two blocks ahead it is warp 3's where that has no T.
+      const int q = 32 + (lane & ~3), i = ph + (warp == 2 ? 1 : 2), c = 16 * i + 4 * (lane & 3);
+      update_blocks<4, false>(S + q * kD64Ld + c, Lt + q, Lt + c, INVERT ? 0 : ph - 1, ph);
+    } else if (INVERT && warp > 0 && warp < 4 && ph > 0) {
+      // T, a row of T^T per column: warp 3 has columns 0..15, warp 1 16..31,
+      // warp 2 32..63 (f: the first block row that is not zero).  Block row
+      // ph - 1 is final once substituted against diagonal block ph - 1; below
+      // row 32, columns 0..31 stop at -W.
+      const int f = warp == 3 ? 0 : warp;
+      const int own = warp == 2 ? lane : lane & 15;
+      float* t = TT + 16 * f * kD64Ld;
+      if (f == 2 || ph < 3) {
+        float* trow = t + own * kD64Ld + 16 * (ph - 1);
+        load_row16(x, trow);
+        subst16(x, Lt + 16 * (ph - 1) * (kD64Ld + 1), sm.invd + 16 * (ph - 1));
+        if (own == lane) store_row16(trow, x);
+        __syncwarp();
+      }
+      // What is final, applied to block row ph; warp 3 takes panel 0's part
+      // of block row ph + 1 a phase early.
+      const int q = 2 * (lane >> 2), g = 4 * (lane & 3);
+      const int jobs = ph == 4 ? 0 : (f == 0 && ph < 3 ? 2 : 1);
+#pragma unroll 1
+      for (int j = 0; j < jobs; ++j) {
+        const int c = 16 * (ph + j) + g;
+        const int k = j == 1 ? 0 : (ph == 3 ? max(f, 1) : ph - 1);
+        update_blocks<2, true>(t + q * kD64Ld + c, t + q * kD64Ld, Lt + c, k, k + 1);
+      }
+    } else if (INVERT && warp == 3) {
+      // T^T starts as the identity.
+#pragma unroll 4
+      for (int e = lane; e < 64 * 16; e += 32) {
+        const int r = e >> 4, c = (e & 15) * 4;
+        *reinterpret_cast<float4*>(TT + r * kD64Ld + c) =
+            make_float4(c == r ? 1.f : 0.f, c + 1 == r ? 1.f : 0.f, c + 2 == r ? 1.f : 0.f, c + 3 == r ? 1.f : 0.f);
+      }
+    }
+    bar();
+    if (warp == 0 && lane < 16 && ph < 4) store_row16(row, x);
+  }
+  if (INVERT && tid < kD64Threads) {
+    // T21^T = -W^T T22^T in place (the four threads of a row are one warp's).
+    const int c = tid >> 2, i0 = 32 + (tid & 3) * 8;
+    float acc[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc[q] = 0.0f;
+#pragma unroll 2
+    for (int p = 0; p < 32; p += 4) {
+      const float4 w4 = *reinterpret_cast<const float4*>(TT + c * kD64Ld + 32 + p);
+      const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float4 b0 = *reinterpret_cast<const float4*>(TT + (32 + p + e) * kD64Ld + i0);
+        const float4 b1 = *reinterpret_cast<const float4*>(TT + (32 + p + e) * kD64Ld + i0 + 4);
+        acc[0] = fmaf(w[e], b0.x, acc[0]);
+        acc[1] = fmaf(w[e], b0.y, acc[1]);
+        acc[2] = fmaf(w[e], b0.z, acc[2]);
+        acc[3] = fmaf(w[e], b0.w, acc[3]);
+        acc[4] = fmaf(w[e], b1.x, acc[4]);
+        acc[5] = fmaf(w[e], b1.y, acc[5]);
+        acc[6] = fmaf(w[e], b1.z, acc[6]);
+        acc[7] = fmaf(w[e], b1.w, acc[7]);
+      }
+    }
+    __syncwarp();
+    float* o = TT + c * kD64Ld + i0;
+    reinterpret_cast<float4*>(o)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    reinterpret_cast<float4*>(o)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  }
+  bar();
+  return diag64_status(sm);
+}
+
+// Factor the block in sm.S (lower triangle and diagonal read; the caller has
+// filled it).  On return sm.S holds L in its lower triangle (what is above the
+// diagonal is unspecified), the L^T view holds Lt[m][j] = L[j][m] for j >= m
+// (other entries unspecified) and sm.invd 1/diag(L).  Returns the first bad
+// pivot or -1.  Every thread of the CTA calls it; threads beyond the first
+// four warps only take part in the barriers.
+template <class Bar = CtaBarrier>
+__device__ __forceinline__ int diag64_factor(Diag64Smem& sm, Bar bar = Bar()) {
+  return diag64_run<false>(sm, bar);
 }
 
 // Column c of L^{-1} for a 32x32 lower L given as lt = L^T (row stride LD)
@@ -277,84 +395,12 @@ __device__ __forceinline__ void col_inverse32(float (&y)[32], int c, const float
   }
 }
 
-// diag64_factor, then T = L^{-1} stored transposed in sm.T:
-// sm.T[c * kD64Ld + j] = T[j][c] (0 for j < c).  W^T is staged in the
-// (zero) lower-left quarter of sm.T and cleared again.
+// diag64_factor, and T = L^{-1} stored transposed in sm.T:
+// sm.T[c * kD64Ld + j] = T[j][c] (0 for j < c).  Threads beyond the first four
+// warps only take part in the barriers.
 template <class Bar = CtaBarrier>
 __device__ __forceinline__ int diag64_factor_invert(Diag64Smem& sm, Bar bar = Bar()) {
-  const int bad = diag64_factor(sm, bar);
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int warp = tid >> 5;
-  const bool active = tid < kD64Threads;
-  const float* Lt = diag64_lt(sm);
-  float* TT = sm.T;
-  if (warp < 2) {
-    // T11 (warp 0) / T22 (warp 1) column `lane` -> row of T^T.
-    float y[32];
-    col_inverse32<kD64Ld>(y, lane, Lt + warp * 32 * (kD64Ld + 1), sm.invd + 32 * warp);
-    float* row = TT + (32 * warp + lane) * kD64Ld + 32 * warp;
-#pragma unroll
-    for (int c4 = 0; c4 < 8; ++c4)
-      reinterpret_cast<float4*>(row)[c4] = make_float4(y[4 * c4], y[4 * c4 + 1], y[4 * c4 + 2], y[4 * c4 + 3]);
-  }
-  bar();
-  const int c = tid >> 2, i0 = (tid & 3) * 8;
-  if (active) {
-    // W^T[c][i] = sum_m T11[m][c] L21[i][m]  (W = L21 T11), into TT[32 + c][i].
-    float acc[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) acc[q] = 0.0f;
-#pragma unroll 8
-    for (int m = 0; m < 32; ++m) {
-      const float a = TT[c * kD64Ld + m];
-      const float4 b0 = *reinterpret_cast<const float4*>(Lt + m * kD64Ld + 32 + i0);
-      const float4 b1 = *reinterpret_cast<const float4*>(Lt + m * kD64Ld + 36 + i0);
-      acc[0] = fmaf(a, b0.x, acc[0]);
-      acc[1] = fmaf(a, b0.y, acc[1]);
-      acc[2] = fmaf(a, b0.z, acc[2]);
-      acc[3] = fmaf(a, b0.w, acc[3]);
-      acc[4] = fmaf(a, b1.x, acc[4]);
-      acc[5] = fmaf(a, b1.y, acc[5]);
-      acc[6] = fmaf(a, b1.z, acc[6]);
-      acc[7] = fmaf(a, b1.w, acc[7]);
-    }
-    float* w = TT + (32 + c) * kD64Ld + i0;
-    reinterpret_cast<float4*>(w)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    reinterpret_cast<float4*>(w)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
-  }
-  bar();
-  if (active) {
-    // T21^T[c][i] = -sum_p W^T[c][p] T22^T[p][i]  (T21 = -T22 W), into TT[c][32 + i].
-    float acc[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) acc[q] = 0.0f;
-#pragma unroll 8
-    for (int p = 0; p < 32; ++p) {
-      const float a = TT[(32 + c) * kD64Ld + p];
-      const float4 b0 = *reinterpret_cast<const float4*>(TT + (32 + p) * kD64Ld + 32 + i0);
-      const float4 b1 = *reinterpret_cast<const float4*>(TT + (32 + p) * kD64Ld + 36 + i0);
-      acc[0] = fmaf(a, b0.x, acc[0]);
-      acc[1] = fmaf(a, b0.y, acc[1]);
-      acc[2] = fmaf(a, b0.z, acc[2]);
-      acc[3] = fmaf(a, b0.w, acc[3]);
-      acc[4] = fmaf(a, b1.x, acc[4]);
-      acc[5] = fmaf(a, b1.y, acc[5]);
-      acc[6] = fmaf(a, b1.z, acc[6]);
-      acc[7] = fmaf(a, b1.w, acc[7]);
-    }
-    float* o = TT + c * kD64Ld + 32 + i0;
-    reinterpret_cast<float4*>(o)[0] = make_float4(-acc[0], -acc[1], -acc[2], -acc[3]);
-    reinterpret_cast<float4*>(o)[1] = make_float4(-acc[4], -acc[5], -acc[6], -acc[7]);
-  }
-  bar();
-  if (active) {
-    float* z = TT + (32 + c) * kD64Ld + i0;
-    reinterpret_cast<float4*>(z)[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-    reinterpret_cast<float4*>(z)[1] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  bar();
-  return bad;
+  return diag64_run<true>(sm, bar);
 }
 
 // Solve one panel row against the factored 64x64 block: x <- x L^{-T}

@@ -143,9 +143,7 @@ __global__ void __launch_bounds__(kD64Threads, 3)
       reinterpret_cast<float4*>(tb)[e4] = v;
     }
     if (info != nullptr && tid == 0) {
-      if (bad == kDiagTimeout)
-        info[tg.mat] = -1;
-      else if (k0 == 0)
+      if (k0 == 0)
         info[tg.mat] = bad >= 0 ? bad + 1 : 0;
       else if (bad >= 0 && info[tg.mat] == 0)
         info[tg.mat] = k0 + bad + 1;

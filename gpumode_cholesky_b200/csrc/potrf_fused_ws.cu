@@ -385,7 +385,7 @@ __device__ void ws_consumers(const WsBars& br, uint8_t* sm, const float* a, floa
           cbar();
           umma::fence_after_sync();
           const int bad = diag64_status(dg);
-          if (bad == kDiagTimeout || *br.flag) {
+          if (*br.flag) {
             failed = true;
             if (tid == 0) *br.flag = 1;  // the producer gives up too
           }

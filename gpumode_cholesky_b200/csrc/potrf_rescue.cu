@@ -143,9 +143,7 @@ __global__ void __launch_bounds__(kRThreads, 1)
                             c + 3 <= r ? srow[3] : 0.f);
           }
           if (tid == 0 && info != nullptr) {
-            if (bad == kDiagTimeout)
-              info[b] = -1;
-            else if (k == 0)
+            if (k == 0)
               info[b] = bad >= 0 ? bad + 1 : 0;
             else if (bad >= 0 && info[b] == 0)
               info[b] = k0 + bad + 1;
