@@ -8,7 +8,8 @@
 //                many CTAs per matrix when n > 1024 or the batch is too
 //                small to fill the GPU one CTA per matrix (potrf_split);
 //                else one CTA per matrix (potrf_fused / potrf_fused_ws);
-//              FP32 or any other n: blocked right-looking (potrf_blocked)
+//              FP32: tile tasks in one launch (potrf_tiles); any other n or
+//              FP64 diagonal tiles: blocked right-looking (potrf_blocked)
 // There is no CPU path and no vendor-library fallback.
 #include <cstdarg>
 #include <cstdio>
@@ -85,7 +86,8 @@ bool path_supported(int path, int64_t batch, int64_t n, int mode) {
 // B200 (BF16x3): up to n = 1024 one CTA per matrix while the batch fills
 // the GPU (640x512: 1225 us), else the warp-specialized kernel in clusters of
 // up to 8 CTAs per matrix (60x1024: 646 us, 4x1024: 421 us); above 1024 the
-// multi-CTA split path (8x2048: 1351 us).  FP32: blocked.
+// multi-CTA split path (8x2048: 1351 us).  FP32: blocked (which is
+// potrf_tiles but for FP64 diagonal tiles).
 int choose_path(int64_t batch, int64_t n, int mode) {
   const int64_t sms = device_sms();
   if (fused_supported(n, mode)) return batch > sms ? B2P_PATH_FUSED : B2P_PATH_FUSED_WS;

@@ -29,6 +29,11 @@ size_t blocked_workspace_bytes(int64_t batch, int64_t n, int mode);
 int potrf_blocked(const float* a, float* l, int64_t batch, int n, int mode, void* ws,
                   size_t ws_bytes, int32_t* info, cudaStream_t s);
 
+// The plain FP32 form of the same (potrf_tiles.cu): one launch of tile tasks,
+// same workspace (tws) and the same values.
+bool tiles_fits(int64_t batch, int64_t n);
+int potrf_tiles(const float* a, float* l, int64_t batch, int n, float* tws, int32_t* info, cudaStream_t s);
+
 // tcgen05 trailing update, TF32 or BF16x3 (syrk_tc.cu).  Dense: `tiles`
 // lower 128x128 tiles per matrix; ragged: one CTA per item of `sch`.
 int T_tc(int n, int k0);
@@ -153,6 +158,7 @@ enum KernelId {
   kKGpForward,
   kKGpLbar,
   kKRescue,
+  kKTiles,
   kKCount
 };
 
@@ -215,6 +221,7 @@ enum SmemSlot {
   kSlotSplitU2,
   kSlotSplitS2,
   kSlotSplitW2,
+  kSlotTiles,
   kSlotCount
 };
 

@@ -1,4 +1,5 @@
-// Blocked right-looking factorization for n > 128 (plain FP32 SIMT form).
+// Blocked right-looking factorization for n > 128 (SIMT form: FP64 diagonal
+// tiles, the ragged schedule, and plain FP32 beyond potrf_tiles.cu's range).
 //
 // The output buffer holds the working matrix.  For each 64-wide block column
 // k0 three kernels run:
@@ -510,6 +511,13 @@ int potrf_blocked(const float* a, float* l, int64_t batch, int n, int mode, void
   if (ws == nullptr || ws_bytes < need)
     return set_error(B2P_ERR_WORKSPACE, "workspace of %zu bytes required, %zu given", need, ws_bytes);
   float* tws = static_cast<float*>(ws);
+  // Plain FP32 runs as one launch of tile tasks at every size its counters
+  // cover (order 65 000 on); the same values at all of them, faster at every
+  // size measured (us per call, three launches a block column -> tiles):
+  // 2x129 78 -> 48, 40x256 106 -> 81, 50x500 290 -> 172, 640x512 1958 -> 1492,
+  // 60x1024 1418 -> 1000, 2x1023 582 -> 292, 8x2048 1624 -> 884,
+  // 1x8192 10 291 -> 5794.
+  if (!tensor && !f64diag && tiles_fits(batch, n)) return potrf_tiles(a, l, batch, n, tws, info, s);
   const int sms = device_sms();
   const size_t dsmem = sizeof(Diag64Smem);
   if (int st = ensure_smem_attr((const void*)diag_kernel<false>, dsmem, kSlotDiag)) return st;

@@ -29,8 +29,8 @@
 //   * the first call on each device looks up the array's device address with
 //     cudaGetSymbolAddress (a host-side query, no allocation); make that first
 //     call before any stream capture.  The first call that reaches the split
-//     path (tensor modes above order 1024) or the FP32 path with its
-//     look-ahead also creates that path's library-owned streams and events
+//     path (tensor modes above order 1024) or the blocked path with its
+//     look-ahead (FP64 diagonal tiles) also creates that path's library-owned streams and events
 //     once per device, so warm each path up once outside capture and outside
 //     any region that must not touch the driver;
 //   * the address is cached per device ordinal: after cudaDeviceReset (or
