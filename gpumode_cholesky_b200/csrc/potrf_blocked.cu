@@ -512,11 +512,11 @@ int potrf_blocked(const float* a, float* l, int64_t batch, int n, int mode, void
     return set_error(B2P_ERR_WORKSPACE, "workspace of %zu bytes required, %zu given", need, ws_bytes);
   float* tws = static_cast<float*>(ws);
   // Plain FP32 runs as one launch of tile tasks at every size its counters
-  // cover (order 65 000 on); the same values at all of them, faster at every
-  // size measured (us per call, three launches a block column -> tiles):
-  // 2x129 78 -> 48, 40x256 106 -> 81, 50x500 290 -> 172, 640x512 1958 -> 1492,
-  // 60x1024 1418 -> 1000, 2x1023 582 -> 292, 8x2048 1624 -> 884,
-  // 1x8192 10 291 -> 5794.
+  // cover (orders up to 65 000); the same values at all of them, faster at
+  // every size measured (us per call, three launches a block column -> tiles):
+  // 2x129 78 -> 44, 64x256 115 -> 76, 50x500 290 -> 158, 640x512 1958 -> 1212,
+  // 60x1024 1418 -> 707, 2x1023 582 -> 251, 8x2048 1624 -> 775,
+  // 1x8192 10 291 -> 5084.
   if (!tensor && !f64diag && tiles_fits(batch, n)) return potrf_tiles(a, l, batch, n, tws, info, s);
   const int sms = device_sms();
   const size_t dsmem = sizeof(Diag64Smem);
