@@ -7,8 +7,11 @@
 // warp w -> the column groups {4w..4w+3} (m < 4w+4) and {60-4w..63-4w}
 // (m < 64-4w), which balances the triangle at 68 K-steps per warp.  PtT is
 // overwritten with X^T (XT[c][r] = X[r][c]) once every warp has finished
-// reading it; `bar` synchronises the 256 threads.
+// reading it; `bar` synchronises the 256 threads.  Rows go in pairs through
+// packed multiply-adds (a lane's four rows of one m are one vector load).
 #pragma once
+
+#include "common.cuh"
 
 namespace b2p {
 
@@ -17,7 +20,7 @@ __device__ __forceinline__ void xgemm_tri_inplace(float* PtT, int ld, const floa
   const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 7;
   const int cA = 4 * w, cB = 60 - 4 * w;
   const int mA = 4 * w + 4, mB = 64 - 4 * w;
-  float accA[4][4], accB[4][4];
+  float accA[4][4], accB[4][4];  // [column][row]
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -27,35 +30,34 @@ __device__ __forceinline__ void xgemm_tri_inplace(float* PtT, int ld, const floa
     const float4 a = *reinterpret_cast<const float4*>(PtT + m * ld + 4 * lane);
     const float4 ba = *reinterpret_cast<const float4*>(TT + m * ldt + cA);
     const float4 bb = *reinterpret_cast<const float4*>(TT + m * ldt + cB);
-    const float a4[4] = {a.x, a.y, a.z, a.w};
     const float b4a[4] = {ba.x, ba.y, ba.z, ba.w};
     const float b4b[4] = {bb.x, bb.y, bb.z, bb.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        accA[i][j] = fmaf(a4[i], b4a[j], accA[i][j]);
-        accB[i][j] = fmaf(a4[i], b4b[j], accB[i][j]);
-      }
+    for (int j = 0; j < 4; ++j) {
+      fma2(accA[j][0], accA[j][1], b4a[j], a.x, a.y);
+      fma2(accA[j][2], accA[j][3], b4a[j], a.z, a.w);
+      fma2(accB[j][0], accB[j][1], b4b[j], a.x, a.y);
+      fma2(accB[j][2], accB[j][3], b4b[j], a.z, a.w);
+    }
   }
 #pragma unroll 4
   for (int m = mA; m < mB; ++m) {
     const float4 a = *reinterpret_cast<const float4*>(PtT + m * ld + 4 * lane);
     const float4 bb = *reinterpret_cast<const float4*>(TT + m * ldt + cB);
-    const float a4[4] = {a.x, a.y, a.z, a.w};
     const float b4b[4] = {bb.x, bb.y, bb.z, bb.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) accB[i][j] = fmaf(a4[i], b4b[j], accB[i][j]);
+    for (int j = 0; j < 4; ++j) {
+      fma2(accB[j][0], accB[j][1], b4b[j], a.x, a.y);
+      fma2(accB[j][2], accB[j][3], b4b[j], a.z, a.w);
+    }
   }
   bar();
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     *reinterpret_cast<float4*>(PtT + (cA + j) * ld + 4 * lane) =
-        make_float4(accA[0][j], accA[1][j], accA[2][j], accA[3][j]);
+        make_float4(accA[j][0], accA[j][1], accA[j][2], accA[j][3]);
     *reinterpret_cast<float4*>(PtT + (cB + j) * ld + 4 * lane) =
-        make_float4(accB[0][j], accB[1][j], accB[2][j], accB[3][j]);
+        make_float4(accB[j][0], accB[j][1], accB[j][2], accB[j][3]);
   }
   bar();
 }
