@@ -97,9 +97,9 @@ __device__ __forceinline__ void store_row16(float* dst, const float (&x)[16]) {
 // The rank-16 update in register tiles of R rows by 4 columns, x[4r + c] -=
 // sum_m a_rm lt[m][c0 + c], m = 0..15 ascending.  The columns' factors come
 // from the L^T view, where a warp's reads of one m are contiguous; so do the
-// rows' (`lt_r`, a_rm = lt_r[m][r]) or, for T, they are rows of T^T (`tt`,
-// a_rm = tt[r][m]).
-template <int R, bool TROWS>
+// rows' (a_rm = rows[m][r]) or they are rows of S or T^T (TROWS, a_rm =
+// rows[r][m]).  SUM: x += instead, in packed pairs.
+template <int R, bool TROWS, bool SUM>
 __device__ __forceinline__ void update_tile16(float (&x)[4 * R], const float* rows, const float* lt_c) {
 #pragma unroll 2
   for (int m = 0; m < 16; m += 4) {
@@ -127,18 +127,24 @@ __device__ __forceinline__ void update_tile16(float (&x)[4 * R], const float* ro
       const float4 b = *reinterpret_cast<const float4*>(lt_c + (m + p) * kD64Ld);
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        x[4 * r + 0] = fmaf(-a[p][r], b.x, x[4 * r + 0]);
-        x[4 * r + 1] = fmaf(-a[p][r], b.y, x[4 * r + 1]);
-        x[4 * r + 2] = fmaf(-a[p][r], b.z, x[4 * r + 2]);
-        x[4 * r + 3] = fmaf(-a[p][r], b.w, x[4 * r + 3]);
+        if (SUM) {
+          fma2(x[4 * r + 0], x[4 * r + 1], a[p][r], b.x, b.y);
+          fma2(x[4 * r + 2], x[4 * r + 3], a[p][r], b.z, b.w);
+        } else {
+          x[4 * r + 0] = fmaf(-a[p][r], b.x, x[4 * r + 0]);
+          x[4 * r + 1] = fmaf(-a[p][r], b.y, x[4 * r + 1]);
+          x[4 * r + 2] = fmaf(-a[p][r], b.z, x[4 * r + 2]);
+          x[4 * r + 3] = fmaf(-a[p][r], b.w, x[4 * r + 3]);
+        }
       }
     }
   }
 }
 
 // The tile's R rows of four at `dst` (row stride kD64Ld), less panels
-// k0 .. k1 - 1 of L (`rows`, `lt_c` as above, at panel 0).
-template <int R, bool TROWS>
+// k0 .. k1 - 1 of L (`rows`, `lt_c` as above, at panel 0): product by product,
+// or with SUM each panel's sum at once.
+template <int R, bool TROWS, bool SUM = false>
 __device__ __forceinline__ void update_blocks(float* dst, const float* rows, const float* lt_c, int k0, int k1) {
   float x[4 * R];
 #pragma unroll
@@ -147,8 +153,19 @@ __device__ __forceinline__ void update_blocks(float* dst, const float* rows, con
     x[4 * r] = v.x, x[4 * r + 1] = v.y, x[4 * r + 2] = v.z, x[4 * r + 3] = v.w;
   }
 #pragma unroll 1
-  for (int k = k0; k < k1; ++k)
-    update_tile16<R, TROWS>(x, rows + 16 * k * (TROWS ? 1 : kD64Ld), lt_c + 16 * k * kD64Ld);
+  for (int k = k0; k < k1; ++k) {
+    const float* rk = rows + 16 * k * (TROWS ? 1 : kD64Ld);
+    if (SUM) {
+      float d[4 * R];
+#pragma unroll
+      for (int q = 0; q < 4 * R; ++q) d[q] = 0.0f;
+      update_tile16<R, TROWS, true>(d, rk, lt_c + 16 * k * kD64Ld);
+#pragma unroll
+      for (int q = 0; q < 4 * R; ++q) x[q] -= d[q];
+    } else {
+      update_tile16<R, TROWS, false>(x, rk, lt_c + 16 * k * kD64Ld);
+    }
+  }
 #pragma unroll
   for (int r = 0; r < R; ++r)
     *reinterpret_cast<float4*>(dst + r * kD64Ld) = make_float4(x[4 * r], x[4 * r + 1], x[4 * r + 2], x[4 * r + 3]);
@@ -241,40 +258,51 @@ __device__ __forceinline__ int diag64_status(const Diag64Smem& sm) {
 }
 
 // The engine's body, see the top of the file; INVERT adds T = L^{-1}.
-// Phase ph (0..3) factors panel ph; with INVERT a phase 4 ends the inverse.
-template <bool INVERT, class Bar>
-__device__ __forceinline__ int diag64_run(Diag64Smem& sm, Bar bar) {
+// Phase ph (0 .. np - 1) factors panel ph; with INVERT a phase 4 ends the
+// inverse.  np < 4 leaves out panels that are identity padding.  BELOW: S has
+// 64 more rows (64 .. 127), which warps 4..7 solve along with the panels, 16
+// rows each; their updates are left-looking, since these warps never run out
+// of panel rows.  SUM: updates subtract a panel's sum at once, which rounds
+// less often at the element's own size (the small orders' form; the n > 128
+// paths keep the product-by-product order).
+template <bool INVERT, bool BELOW, bool SUM, class Bar>
+__device__ __forceinline__ void diag64_panels(float* S, float* Lt, float* TT, float* invd, int* bad, int np,
+                                              Bar bar) {
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
-  float* S = sm.S;
-  float* Lt = diag64_lt(sm);
-  float* TT = sm.T;
+  if (tid == 0)
+    for (int p = np; p < 4; ++p) bad[p] = -1;
 #pragma unroll 1
-  for (int ph = 0; ph < (INVERT ? 5 : 4); ++ph) {
+  for (int ph = 0; ph < (INVERT ? 5 : np); ++ph) {
     if (ph > 0 && ph < 4) {
       // Panel ph - 1 applied to column block ph: rows 16 ph .. 63, two rows
       // and four columns a thread.
       const int r = 16 * ph + 2 * (tid >> 2), c = 16 * ph + 4 * (tid & 3);
-      if (r < 64) update_blocks<2, false>(S + r * kD64Ld + c, Lt + r, Lt + c, ph - 1, ph);
+      if (BELOW && tid >= kD64Threads) {
+        const int rb = 2 * (tid >> 2);  // 64 ..
+        update_blocks<2, true, SUM>(S + rb * kD64Ld + c, S + rb * kD64Ld, Lt + c, 0, ph);
+      } else if (r < 64) {
+        update_blocks<2, false, SUM>(S + r * kD64Ld + c, Lt + r, Lt + c, ph - 1, ph);
+      }
       bar();
     }
     float x[16];
     float* row = nullptr;
-    if (ph < 4 && warp < 3 && (warp + ph < 3 || warp == 0)) {
-      // The panel.  The last one has no rows for lanes 16..31.
-      const int r = 16 * (lane < 16 ? ph : ph + warp) + lane;
-      const bool live = r < 64;
+    if (ph < 4 && ((warp < 3 && (warp + ph < 3 || warp == 0)) || (BELOW && warp >= 4))) {
+      // The panel.  The last one has no rows of the block for lanes 16..31.
+      const int r = 16 * (lane < 16 ? ph : (BELOW && warp >= 4) ? warp - 1 : ph + warp) + lane;
+      const bool live = r < 64 || (BELOW && warp >= 4);
       row = S + (live ? r : 48) * kD64Ld + 16 * ph;
       load_row16(x, row);
-      int b = factor16<true>(x, lane, sm.invd + 16 * ph);
+      int b = factor16<true>(x, lane, invd + 16 * ph);
       if (b != 0) {
         load_row16(x, row);
-        b = factor16<false>(x, lane, sm.invd + 16 * ph);
+        b = factor16<false>(x, lane, invd + 16 * ph);
       } else {
         b = -1;
       }
-      if (tid == 0) sm.bad[ph] = b;
+      if (tid == 0) bad[ph] = b;
       // The diagonal block is warp 0's to write, zero above its diagonal; into
       // S after the barrier, since every panel warp reads it there.
       if (live && (lane >= 16 || warp == 0)) {
@@ -283,15 +311,17 @@ __device__ __forceinline__ int diag64_run(Diag64Smem& sm, Bar bar) {
 #pragma unroll
           for (int c = 0; c < 16; ++c) x[c] = c <= lane ? x[c] : 0.0f;
         }
-        float* lc = Lt + 16 * ph * kD64Ld + r;
+        if (!BELOW || r < 64) {
+          float* lc = Lt + 16 * ph * kD64Ld + r;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) lc[c * kD64Ld] = x[c];
+          for (int c = 0; c < 16; ++c) lc[c * kD64Ld] = x[c];
+        }
       }
     } else if ((warp == 2 && ph < 3) || (!INVERT && warp == 3 && ph == 1)) {
       // Panels before ph applied to the columns beyond block ph: warp 2 one
       // block ahead; two blocks ahead it is warp 3's where that has no T.
       const int q = 32 + (lane & ~3), i = ph + (warp == 2 ? 1 : 2), c = 16 * i + 4 * (lane & 3);
-      update_blocks<4, false>(S + q * kD64Ld + c, Lt + q, Lt + c, INVERT ? 0 : ph - 1, ph);
+      update_blocks<4, false, SUM>(S + q * kD64Ld + c, Lt + q, Lt + c, INVERT ? 0 : ph - 1, ph);
     } else if (INVERT && warp > 0 && warp < 4 && ph > 0) {
       // T, a row of T^T per column: warp 3 has columns 0..15, warp 1 16..31,
       // warp 2 32..63 (f: the first block row that is not zero).  Block row
@@ -303,7 +333,7 @@ __device__ __forceinline__ int diag64_run(Diag64Smem& sm, Bar bar) {
       if (f == 2 || ph < 3) {
         float* trow = t + own * kD64Ld + 16 * (ph - 1);
         load_row16(x, trow);
-        subst16(x, Lt + 16 * (ph - 1) * (kD64Ld + 1), sm.invd + 16 * (ph - 1));
+        subst16(x, Lt + 16 * (ph - 1) * (kD64Ld + 1), invd + 16 * (ph - 1));
         if (own == lane) store_row16(trow, x);
         __syncwarp();
       }
@@ -359,6 +389,11 @@ __device__ __forceinline__ int diag64_run(Diag64Smem& sm, Bar bar) {
     reinterpret_cast<float4*>(o)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
   }
   bar();
+}
+
+template <bool INVERT, class Bar>
+__device__ __forceinline__ int diag64_run(Diag64Smem& sm, Bar bar) {
+  diag64_panels<INVERT, false, false>(sm.S, diag64_lt(sm), sm.T, sm.invd, sm.bad, 4, bar);
   return diag64_status(sm);
 }
 
@@ -405,21 +440,25 @@ __device__ __forceinline__ int diag64_factor_invert(Diag64Smem& sm, Bar bar = Ba
 
 // Solve one panel row against the factored 64x64 block: x <- x L^{-T}
 // (forward substitution, FP32, right-looking over the columns), with L^T as
-// diag64_factor leaves it.  2080 FMAs per row; every shared-memory read is a
-// warp-wide broadcast.
+// diag64_factor leaves it.  2080 multiply-adds per row, in pairs of columns;
+// every shared-memory read is a warp-wide broadcast.
 __device__ __forceinline__ void panel_solve64(float (&x)[64], const Diag64Smem& sm) {
   const float* Lt = diag64_lt(sm);
 #pragma unroll
   for (int m = 0; m < 64; ++m) {
     x[m] *= sm.invd[m];
+    const float nx = -x[m];
 #pragma unroll
     for (int j4 = (m + 1) / 4; j4 < 16; ++j4) {
       const float4 c = reinterpret_cast<const float4*>(Lt + m * kD64Ld)[j4];
       const float cv[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < 4; q += 2) {
         const int j = 4 * j4 + q;
-        if (j > m) x[j] = fmaf(-x[m], cv[q], x[j]);
+        if (j > m)
+          fma2(x[j], x[j + 1], nx, cv[q], cv[q + 1]);
+        else if (j + 1 > m)
+          x[j + 1] = fmaf(nx, cv[q + 1], x[j + 1]);
       }
     }
   }

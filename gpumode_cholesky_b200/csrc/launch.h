@@ -222,6 +222,7 @@ enum SmemSlot {
   kSlotSplitS2,
   kSlotSplitW2,
   kSlotTiles,
+  kSlotCta64,
   kSlotCount
 };
 

@@ -226,8 +226,7 @@ __global__ void __launch_bounds__(kBsThreads, 1)
   float* bB = bsm + kBsBuf;      // Lbar, later P^T, later Z
   float* bC = bsm + 2 * kBsBuf;  // U = L^{-1}
   float* work = bsm + 3 * kBsBuf;
-  TileScratch sc{};
-  sc.invd = work + kBsWork;
+  float* invd = work + kBsWork;
   const int tid = threadIdx.x;
   const int ti = tid >> 5, tj = tid & 31;  // rows 8ti.., columns 4tj..
   float acc[8][4];
@@ -242,7 +241,7 @@ __global__ void __launch_bounds__(kBsThreads, 1)
       bB[i * kBsLd + j] = in ? G[(size_t)i * n + j] : 0.0f;
     }
     __syncthreads();
-    if (tid < 128) sc.invd[tid] = 1.0f / bA[tid * kBsLd + tid];
+    if (tid < 128) invd[tid] = 1.0f / bA[tid * kBsLd + tid];
     // P = Phi(L^T Lbar) (tiles reaching the lower triangle; k >= max(i, j)),
     // kept in registers.
     const bool lower = 4 * tj <= 8 * ti + 7;
@@ -264,7 +263,7 @@ __global__ void __launch_bounds__(kBsThreads, 1)
       dst[1] = make_float4(v[4], v[5], v[6], v[7]);
     }
     // U = L^{-1} into bC.
-    trtri128(bA, bC, kBsLd, sc.invd, work);
+    trtri128(bA, bC, kBsLd, invd, work);
     // Z = P U: Z[i][j] = sum_k P^T[k][i] U[k][j], k in [j, i] (lower tiles).
     if (lower) bs_tile(bB, bC, ti, tj, 4 * tj, 8 * ti + 8, acc);
     __syncthreads();

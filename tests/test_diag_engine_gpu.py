@@ -63,3 +63,26 @@ def test_oracle_agrees_on_the_failing_place():
     a[0, 81, 81] = -1.0
     _, info = oracle.potrf_f64(a.numpy())
     assert int(info[0]) == 82
+
+
+@pytest.mark.parametrize("n", [33, 47, 48, 49, 63, 64, 65, 66, 79, 80, 81, 96, 97, 111, 112, 113, 127, 128])
+def test_small_orders(n):
+    """One CTA per matrix: the edges of its panels, blocks and vector loads."""
+    batch = 5
+    a = inputs.well_conditioned(batch, n, 200 + n, device="cpu")
+    bad = [None, 0, n - 1, 17, 31]
+    for b, k in enumerate(bad):
+        if k is not None:
+            a[b, k, k] = -1.0
+    info = torch.full((batch,), 9, dtype=torch.int32, device="cuda")
+    out = torch.full((batch, n, n), float("nan"), device="cuda")
+    l = cholesky(a.cuda(), info=info, out=out).cpu()
+    assert info.cpu().tolist() == [0 if k is None else k + 1 for k in bad]
+    assert not torch.triu(l, 1).any()
+    l64, _ = oracle.potrf_f64(a[:1].numpy())
+    want = torch.from_numpy(l64)[0]
+    # Eigenvalues of M M^T / n + I lie in [1, 5]: n + 1 roundings, amplified 5 times.
+    assert float(torch.linalg.norm(l[0].double() - want) / torch.linalg.norm(want)) <= 5 * (n + 1) * 2.0**-24
+    for b, k in enumerate(bad):
+        if k is not None:
+            assert torch.isfinite(l[b, :, :k]).all() and torch.isnan(l[b, k:, k]).all()
