@@ -65,20 +65,14 @@ struct NamedBarrier2 {
 
 struct Diag64Smem {
   float S[64 * kD64Ld];   // block: A in, L out (lower part)
-  float T[64 * kD64Ld];   // diag64_factor_invert: T^T, T = L^{-1} (T[c][j] = L^{-1}[j][c])
-  // diag64_factor: L^T viewed as 64 x kD64Ld floats (diag64_lt).
-  // diag64_invert_only: L11^T, L22^T, L21^T and L21 T11 (stride kLtLd).
-  float lt0[32 * kLtLd];
-  float lt1[32 * kLtLd];
-  float p21t[32 * kLtLd];
-  float w21[32 * kLtLd];
+  float T[64 * kD64Ld];   // T^T, T = L^{-1} (T[c][j] = L^{-1}[j][c])
+  float lt[64 * kD64Ld];  // L^T (diag64_lt): lt[m][j] = L[j][m]
   float invd[64];         // 1 / diag(L)
   int bad[4];             // first bad pivot within each panel, or -1
 };
 
-__device__ __forceinline__ float* diag64_lt(Diag64Smem& sm) { return sm.lt0; }
-__device__ __forceinline__ const float* diag64_lt(const Diag64Smem& sm) { return sm.lt0; }
-static_assert(4 * 32 * kLtLd >= 64 * kD64Ld, "the L^T view must fit lt0..w21");
+__device__ __forceinline__ float* diag64_lt(Diag64Smem& sm) { return sm.lt; }
+__device__ __forceinline__ const float* diag64_lt(const Diag64Smem& sm) { return sm.lt; }
 
 // ---- 16-wide pieces: one row (or one right-hand side) per lane ---------------
 __device__ __forceinline__ void load_row16(float (&x)[16], const float* src) {
@@ -257,6 +251,34 @@ __device__ __forceinline__ int diag64_status(const Diag64Smem& sm) {
   return -1;
 }
 
+// T21^T = -W^T T22^T in place (T^T's rows 0..31, columns 32..63 hold -W^T; the
+// four threads of a row are one warp's).  128 threads.
+__device__ __forceinline__ void t21_product(float* TT) {
+  const int tid = threadIdx.x;
+  const int c = tid >> 2, i0 = 32 + (tid & 3) * 8;
+  float acc[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) acc[q] = 0.0f;
+#pragma unroll 2
+  for (int p = 0; p < 32; p += 4) {
+    const float4 w4 = *reinterpret_cast<const float4*>(TT + c * kD64Ld + 32 + p);
+    const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float4 b0 = *reinterpret_cast<const float4*>(TT + (32 + p + e) * kD64Ld + i0);
+      const float4 b1 = *reinterpret_cast<const float4*>(TT + (32 + p + e) * kD64Ld + i0 + 4);
+      fma2(acc[0], acc[1], w[e], b0.x, b0.y);
+      fma2(acc[2], acc[3], w[e], b0.z, b0.w);
+      fma2(acc[4], acc[5], w[e], b1.x, b1.y);
+      fma2(acc[6], acc[7], w[e], b1.z, b1.w);
+    }
+  }
+  __syncwarp();
+  float* o = TT + c * kD64Ld + i0;
+  reinterpret_cast<float4*>(o)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  reinterpret_cast<float4*>(o)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+}
+
 // The engine's body, see the top of the file; INVERT adds T = L^{-1}.
 // Phase ph (0 .. np - 1) factors panel ph; with INVERT a phase 4 ends the
 // inverse.  np < 4 leaves out panels that are identity padding.  BELOW: S has
@@ -359,35 +381,7 @@ __device__ __forceinline__ void diag64_panels(float* S, float* Lt, float* TT, fl
     bar();
     if (warp == 0 && lane < 16 && ph < 4) store_row16(row, x);
   }
-  if (INVERT && tid < kD64Threads) {
-    // T21^T = -W^T T22^T in place (the four threads of a row are one warp's).
-    const int c = tid >> 2, i0 = 32 + (tid & 3) * 8;
-    float acc[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) acc[q] = 0.0f;
-#pragma unroll 2
-    for (int p = 0; p < 32; p += 4) {
-      const float4 w4 = *reinterpret_cast<const float4*>(TT + c * kD64Ld + 32 + p);
-      const float w[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float4 b0 = *reinterpret_cast<const float4*>(TT + (32 + p + e) * kD64Ld + i0);
-        const float4 b1 = *reinterpret_cast<const float4*>(TT + (32 + p + e) * kD64Ld + i0 + 4);
-        acc[0] = fmaf(w[e], b0.x, acc[0]);
-        acc[1] = fmaf(w[e], b0.y, acc[1]);
-        acc[2] = fmaf(w[e], b0.z, acc[2]);
-        acc[3] = fmaf(w[e], b0.w, acc[3]);
-        acc[4] = fmaf(w[e], b1.x, acc[4]);
-        acc[5] = fmaf(w[e], b1.y, acc[5]);
-        acc[6] = fmaf(w[e], b1.z, acc[6]);
-        acc[7] = fmaf(w[e], b1.w, acc[7]);
-      }
-    }
-    __syncwarp();
-    float* o = TT + c * kD64Ld + i0;
-    reinterpret_cast<float4*>(o)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    reinterpret_cast<float4*>(o)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
-  }
+  if (INVERT && tid < kD64Threads) t21_product(TT);
   bar();
 }
 
@@ -406,28 +400,6 @@ __device__ __forceinline__ int diag64_run(Diag64Smem& sm, Bar bar) {
 template <class Bar = CtaBarrier>
 __device__ __forceinline__ int diag64_factor(Diag64Smem& sm, Bar bar = Bar()) {
   return diag64_run<false>(sm, bar);
-}
-
-// Column c of L^{-1} for a 32x32 lower L given as lt = L^T (row stride LD)
-// and invd = 1/diag: forward substitution L y = e_c in right-looking order.
-template <int LD>
-__device__ __forceinline__ void col_inverse32(float (&y)[32], int c, const float* lt, const float* invd) {
-#pragma unroll
-  for (int j = 0; j < 32; ++j) y[j] = (j == c) ? 1.0f : 0.0f;
-#pragma unroll
-  for (int m = 0; m < 32; ++m) {
-    y[m] *= invd[m];
-#pragma unroll
-    for (int j4 = (m + 1) / 4; j4 < 8; ++j4) {
-      const float4 cc = reinterpret_cast<const float4*>(lt + m * LD)[j4];
-      const float cv[4] = {cc.x, cc.y, cc.z, cc.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int j = 4 * j4 + e;
-        if (j > m) y[j] = fmaf(-cv[e], y[m], y[j]);
-      }
-    }
-  }
 }
 
 // diag64_factor, and T = L^{-1} stored transposed in sm.T:
@@ -464,73 +436,47 @@ __device__ __forceinline__ void panel_solve64(float (&x)[64], const Diag64Smem& 
   }
 }
 
-// Inverse only: T = L^{-1} (row-major in sm.T) of the lower-triangular 64x64
-// block already in sm.S (diagonal and lower part valid; identity padding
-// beyond the true width).  Uses lt0/lt1/p21t/w21 as scratch.  All threads
-// call it.
-template <class Bar = CtaBarrier>
-__device__ __forceinline__ void diag64_invert_only(Diag64Smem& sm, Bar bar = Bar()) {
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int warp = tid >> 5;
-  const bool active = tid < kD64Threads;
-  if (active) {
-    for (int e = tid; e < 64 * kD64Ld; e += kD64Threads) sm.T[e] = 0.0f;
-    // L11^T, L22^T, L21^T and 1/diag.
-    for (int e = tid; e < 1024; e += kD64Threads) {
-      const int r = e >> 5, c = e & 31;
-      sm.lt0[c * kLtLd + r] = (c <= r) ? sm.S[r * kD64Ld + c] : 0.0f;
-      sm.lt1[c * kLtLd + r] = (c <= r) ? sm.S[(32 + r) * kD64Ld + 32 + c] : 0.0f;
-      sm.p21t[c * kLtLd + r] = sm.S[(32 + r) * kD64Ld + c];
-    }
-    if (tid < 64) sm.invd[tid] = 1.0f / sm.S[tid * kD64Ld + tid];
+// Inverse only: T = L^{-1} stored transposed in sm.T like diag64_factor_invert,
+// of the lower-triangular 64x64 block in sm.S (identity padding beyond the
+// true width; zero above the diagonal), with L^T already in the L^T view.
+// 128 threads.
+__device__ __forceinline__ void diag64_invert_only(Diag64Smem& sm) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const float* Lt = diag64_lt(sm);
+  float* TT = sm.T;
+  if (tid < 64) sm.invd[tid] = 1.0f / sm.S[tid * kD64Ld + tid];
+  for (int e = tid; e < 64 * 16; e += kD64Threads) {
+    const int r = e >> 4, c = (e & 15) * 4;
+    *reinterpret_cast<float4*>(TT + r * kD64Ld + c) =
+        make_float4(c == r ? 1.f : 0.f, c + 1 == r ? 1.f : 0.f, c + 2 == r ? 1.f : 0.f, c + 3 == r ? 1.f : 0.f);
   }
-  bar();
-  if (warp == 0) {
-    float y[32];
-    col_inverse32<kLtLd>(y, lane, sm.lt0, sm.invd);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) sm.T[j * kD64Ld + lane] = y[j];
-  } else if (warp == 1) {
-    float y[32];
-    col_inverse32<kLtLd>(y, lane, sm.lt1, sm.invd + 32);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) sm.T[(32 + j) * kD64Ld + 32 + lane] = y[j];
+  __syncthreads();
+  // Warp w: columns 16w .. 16w + 15, T11 and T22.
+  const int h = 2 * (warp >> 1);  // the half's first block row
+  const int q = 2 * (lane >> 2), g = 4 * (lane & 3);
+  float* t = TT + 16 * warp * kD64Ld;
+  float* trow = t + (lane & 15) * kD64Ld;
+  float x[16];
+#pragma unroll 1
+  for (int i = warp; i < h + 2; ++i) {
+    load_row16(x, trow + 16 * i);
+    subst16(x, Lt + 16 * i * (kD64Ld + 1), sm.invd + 16 * i);
+    if (lane < 16) store_row16(trow + 16 * i, x);
+    __syncwarp();
+    if (i == h)
+      update_blocks<2, true>(t + q * kD64Ld + 16 * (i + 1) + g, t + q * kD64Ld, Lt + 16 * (i + 1) + g, i, i + 1);
+    __syncwarp();
   }
-  bar();
-  if (active) {
-    // W = L21 T11: thread -> row i, 8 columns.
-    const int i = tid >> 2, c0 = (tid & 3) * 8;
-    float sacc[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) sacc[q] = 0.0f;
-    for (int m = 0; m < 32; ++m) {
-      const float a = sm.p21t[m * kLtLd + i];
-      const float* trow = sm.T + m * kD64Ld + c0;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) sacc[q] = fmaf(a, trow[q], sacc[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) sm.w21[i * kLtLd + c0 + q] = sacc[q];
+  __syncthreads();
+  // -W (W = L21 T11): block row 2 on warps 0 and 1, 3 on 2 and 3.
+  {
+    const int c = 16 * (2 + (warp >> 1)) + g;
+    float* tw = TT + (16 * (warp & 1) + q) * kD64Ld;
+    update_blocks<2, true>(tw + c, tw, Lt + c, 0, 2);
   }
-  bar();
-  if (active) {
-    // T21 = -T22 W.
-    const int i = tid >> 2, c0 = (tid & 3) * 8;
-    float sacc[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) sacc[q] = 0.0f;
-    const float* trow = sm.T + (32 + i) * kD64Ld + 32;
-    for (int m = 0; m <= i; ++m) {
-      const float a = trow[m];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) sacc[q] = fmaf(a, sm.w21[m * kLtLd + c0 + q], sacc[q]);
-    }
-    float* out = sm.T + (32 + i) * kD64Ld + c0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) out[q] = -sacc[q];
-  }
-  bar();
+  __syncthreads();
+  t21_product(TT);
+  __syncthreads();
 }
 
 }  // namespace b2p

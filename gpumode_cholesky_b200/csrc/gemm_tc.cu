@@ -8,10 +8,14 @@
 // parts of K where an operand is known to be zero (triangular operands), skip
 // tiles strictly above the diagonal when only the lower triangle of C is
 // wanted, and apply Phi (keep the lower triangle, halve the diagonal) in the
-// epilogue.  One 128-thread CTA per output tile: per 64-wide K chunk every
+// epilogue.  One 256-thread CTA per output tile: per 64-wide K chunk every
 // thread stages one operand row (128B-swizzled K-major, BF16 hi/lo split or
 // TF32), thread 0 issues the MMAs into a 128x128 FP32 TMEM accumulator, and
 // the epilogue reads TMEM with tcgen05.ld.  Waits are bounded.
+//
+// A triangular hint also means that the other triangle is not read: elements
+// there count as zero whatever the memory holds, so the adjoint's scratch
+// matrices need no clearing.
 #include <algorithm>
 
 #include "launch.h"
@@ -21,7 +25,7 @@ namespace b2p {
 
 constexpr int kGT = 128;  // tile edge
 constexpr int kGK = 64;   // K chunk
-constexpr int kGThreads = 128;
+constexpr int kGThreads = 256;  // 128 stage the A rows, 128 the B rows; all run the epilogue
 constexpr uint32_t kGPolls = 1u << 24;
 constexpr size_t kGOperand = 32768;
 constexpr size_t kGSmem = 2 * kGOperand + 1024 + 64;
@@ -62,18 +66,29 @@ __device__ __forceinline__ void g_store_row(uint8_t* op, int r, const float (&v)
   }
 }
 
+// Which elements (row i, inner k) of an operand its triangular hint keeps.
+enum Keep { kKeepAll = 0, kKeepUpTo = 1 /* k <= i */, kKeepFrom = 2 /* k >= i */ };
+__host__ __device__ __forceinline__ int keep_x(int x_tri) { return x_tri; }
+__host__ __device__ __forceinline__ int keep_y(int y_tri) { return y_tri == 1 ? kKeepFrom : (y_tri == 2 ? kKeepUpTo : kKeepAll); }
+// The part [lo, hi) of k0 .. k0 + len - 1 (relative to k0) that exists and is
+// kept in row i.
+__device__ __forceinline__ int2 kept_range(int keep, int i, int rows, int k0, int kdim, int len) {
+  const int lo = keep == kKeepFrom ? max(0, i - k0) : 0;
+  const int hi = i >= rows ? 0 : min(min(len, kdim - k0), keep == kKeepUpTo ? i - k0 + 1 : len);
+  return make_int2(lo, hi);
+}
 // Operand row `r` (0..127) of a tile: logical element (row0 + r, k0 + kk).
 // `rowmajor`: element (i, kk) at mat[i*ld + kk] (K contiguous) else at
 // mat[kk*ld + i] (rows contiguous across threads: coalesced).
 template <int MODE>
-__device__ __forceinline__ void g_stage(const float* mat, int ld, bool rowmajor, int rows, int kdim, int row0,
-                                        int k0, uint8_t* op, int r) {
+__device__ __forceinline__ void g_stage(const float* mat, int ld, bool rowmajor, int keep, int rows, int kdim,
+                                        int row0, int k0, uint8_t* op, int r) {
   float v[64];
   const int i = row0 + r;
+  const int2 in = kept_range(keep, i, rows, k0, kdim, kGK);
   if (rowmajor) {
     const float* p = mat + (size_t)i * ld + k0;
-    const bool full = (i < rows) && (k0 + kGK <= kdim) && ((ld & 3) == 0);
-    if (full) {
+    if (in.x == 0 && in.y == kGK && (ld & 3) == 0) {
 #pragma unroll
       for (int q = 0; q < 16; ++q) {
         const float4 t = reinterpret_cast<const float4*>(p)[q];
@@ -84,14 +99,41 @@ __device__ __forceinline__ void g_stage(const float* mat, int ld, bool rowmajor,
       }
     } else {
 #pragma unroll
-      for (int q = 0; q < 64; ++q) v[q] = (i < rows && k0 + q < kdim) ? p[q] : 0.0f;
+      for (int q = 0; q < 64; ++q) v[q] = (q >= in.x && q < in.y) ? p[q] : 0.0f;
     }
   } else {
     const float* p = mat + (size_t)k0 * ld + i;
 #pragma unroll
-    for (int q = 0; q < 64; ++q) v[q] = (i < rows && k0 + q < kdim) ? p[(size_t)q * ld] : 0.0f;
+    for (int q = 0; q < 64; ++q) v[q] = (q >= in.x && q < in.y) ? p[(size_t)q * ld] : 0.0f;
   }
   g_store_row<MODE>(op, r, v);
+}
+
+// Row i, columns j0 .. j0 + 31 of the output.
+__device__ __forceinline__ void g_store_out(const GemmArgs& g, float* C, const float* Cin, int i, int j0,
+                                            const float (&v)[32]) {
+  if (i >= g.m) return;
+  float* crow = C + (size_t)i * g.ldc + j0;
+  // A whole run away from the diagonal goes out as vectors.
+  if (g.beta == 0.0f && j0 + 31 < g.n && (!(g.lower_out || g.phi) || j0 + 31 < i) &&
+      (reinterpret_cast<uintptr_t>(crow) & 15u) == 0) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      reinterpret_cast<float4*>(crow)[q] = make_float4(g.alpha * v[4 * q], g.alpha * v[4 * q + 1],
+                                                       g.alpha * v[4 * q + 2], g.alpha * v[4 * q + 3]);
+    return;
+  }
+  const float* cin = Cin + (size_t)i * g.ldc + j0;
+#pragma unroll
+  for (int e = 0; e < 32; ++e) {
+    const int j = j0 + e;
+    if (j < g.n && (!g.lower_out || j <= i)) {
+      float r = g.alpha * v[e];
+      if (g.phi) r = (j > i) ? 0.0f : (j == i ? 0.5f * r : r);
+      if (g.beta != 0.0f) r += g.beta * cin[e];
+      crow[e] = r;
+    }
+  }
 }
 
 template <int MODE>
@@ -175,8 +217,10 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_tc_kernel(GemmArgs g, int t
     bool any = false;
     for (int k0 = klo; k0 < khi; k0 += kGK) {
       // A operand: rows m (op1(X)[m][k]); B operand: rows n (op2(Y)[k][n]).
-      g_stage<MODE>(X, g.ldx, !g.trans_x, g.m, g.k, m0, k0, opA, tid);
-      g_stage<MODE>(Y, g.ldy, g.trans_y, g.n, g.k, n0, k0, opB, tid);
+      const bool xs = tid < kGT;
+      g_stage<MODE>(xs ? X : Y, xs ? g.ldx : g.ldy, xs ? !g.trans_x : g.trans_y != 0,
+                    xs ? keep_x(g.x_tri) : keep_y(g.y_tri), xs ? g.m : g.n, g.k, xs ? m0 : n0, k0, xs ? opA : opB,
+                    tid & (kGT - 1));
       umma::fence_proxy_async_smem();
       umma::fence_before_sync();
       __syncthreads();
@@ -197,31 +241,18 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_tc_kernel(GemmArgs g, int t
       any = true;
     }
     if (!ok) break;
-    // Epilogue: row i = m0 + 32*warp + lane, 4 chunks of 32 columns.
-    const int i = m0 + 32 * warp + lane;
+    // Epilogue: row i = m0 + 32 (warp % 4) + lane, two chunks of 32 columns.
+    const int wq = warp & 3;
 #pragma unroll 1
-    for (int ch = 0; ch < 4; ++ch) {
+    for (int ch = 2 * (warp >> 2); ch < 2 * (warp >> 2) + 2; ++ch) {
       float v[32];
       if (any) {
-        umma::tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(32 * ch), v);
+        umma::tmem_ld32(tmem + ((uint32_t)(32 * wq) << 16) + (uint32_t)(32 * ch), v);
       } else {
 #pragma unroll
         for (int e = 0; e < 32; ++e) v[e] = 0.0f;
       }
-      if (i < g.m) {
-        float* crow = C + (size_t)i * g.ldc;
-        const float* cin = Cin + (size_t)i * g.ldc;
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          const int j = n0 + 32 * ch + e;
-          if (j < g.n && (!g.lower_out || j <= i)) {
-            float r = g.alpha * v[e];
-            if (g.phi) r = (j > i) ? 0.0f : (j == i ? 0.5f * r : r);
-            if (g.beta != 0.0f) r += g.beta * cin[j];
-            crow[j] = r;
-          }
-        }
-      }
+      g_store_out(g, C, Cin, m0 + 32 * wq + lane, n0 + 32 * ch, v);
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -254,9 +285,13 @@ constexpr int kPThreads = 512;
 
 template <int MODE>
 __global__ void __launch_bounds__(kPThreads) gemm_pack_kernel(const float* __restrict__ mat, int64_t s1, int64_t s2,
-                                                              int64_t nb2, int ld, int rowmajor, int rows, int kdim,
-                                                              int tiles_k, int64_t items, uint8_t* __restrict__ out) {
+                                                              int64_t nb2, int ld, int rowmajor, int keep, int rows,
+                                                              int kdim, int tiles_k, int64_t items,
+                                                              uint8_t* __restrict__ out) {
   const int tr = blockIdx.x / tiles_k, tk = blockIdx.x - (blockIdx.x / tiles_k) * tiles_k;
+  // Blocks wholly in the triangle the hint leaves out are not read by the product.
+  if (keep == kKeepUpTo && tk * kGK > tr * kGT + kGT - 1) return;
+  if (keep == kKeepFrom && tk * kGK + kGK - 1 < tr * kGT) return;
   const int r = threadIdx.x & 127, p = threadIdx.x >> 7;
   const int i = tr * kGT + r, k0 = tk * kGK + 16 * p;
   const size_t per = (size_t)((rows + kGT - 1) / kGT) * tiles_k * kGOperand;
@@ -264,9 +299,10 @@ __global__ void __launch_bounds__(kPThreads) gemm_pack_kernel(const float* __res
     const int64_t b1 = b / nb2, b2 = b - (b / nb2) * nb2;
     const float* M = mat + b1 * s1 + b2 * s2;
     float v[16];
+    const int2 in = kept_range(keep, i, rows, k0, kdim, 16);
     if (rowmajor) {
       const float* src = M + (size_t)i * ld + k0;
-      if (i < rows && k0 + 16 <= kdim && ((reinterpret_cast<uintptr_t>(src) & 15u) == 0)) {
+      if (in.x == 0 && in.y == 16 && ((reinterpret_cast<uintptr_t>(src) & 15u) == 0)) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const float4 t = __ldg(reinterpret_cast<const float4*>(src) + q);
@@ -277,11 +313,11 @@ __global__ void __launch_bounds__(kPThreads) gemm_pack_kernel(const float* __res
         }
       } else {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) v[q] = (i < rows && k0 + q < kdim) ? __ldg(src + q) : 0.0f;
+        for (int q = 0; q < 16; ++q) v[q] = (q >= in.x && q < in.y) ? __ldg(src + q) : 0.0f;
       }
     } else {
 #pragma unroll
-      for (int q = 0; q < 16; ++q) v[q] = (i < rows && k0 + q < kdim) ? __ldg(M + (size_t)(k0 + q) * ld + i) : 0.0f;
+      for (int q = 0; q < 16; ++q) v[q] = (q >= in.x && q < in.y) ? __ldg(M + (size_t)(k0 + q) * ld + i) : 0.0f;
     }
     uint8_t* op = out + b * per + (size_t)blockIdx.x * kGOperand;
     if (MODE == B2P_MODE_TF32) {
@@ -480,20 +516,7 @@ __global__ void __launch_bounds__(kBThreads, 1) gemm_bulk_kernel(GemmArgs g, int
 #pragma unroll
           for (int e = 0; e < 32; ++e) v[e] = 0.0f;
         }
-        if (i < g.m) {
-          float* crow = C + (size_t)i * g.ldc;
-          const float* cin = Cin + (size_t)i * g.ldc;
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const int j = t.n0 + 32 * ch + e;
-            if (j < g.n && (!g.lower_out || j <= i)) {
-              float r = g.alpha * v[e];
-              if (g.phi) r = (j > i) ? 0.0f : (j == i ? 0.5f * r : r);
-              if (g.beta != 0.0f) r += g.beta * cin[j];
-              crow[j] = r;
-            }
-          }
-        }
+        g_store_out(g, C, Cin, i, t.n0 + 32 * ch, v);
       }
       umma::fence_before_sync();
       __syncwarp();
@@ -515,10 +538,11 @@ static int launch_gemm_packed(const GemmArgs& g, int32_t* err, cudaStream_t s, i
   const unsigned by = (unsigned)std::min<int64_t>(items, 65535);
   {
     TraceScope ts(kKBwdGemm, s);
-    gemm_pack_kernel<MODE><<<dim3(tm * tk, by), kPThreads, 0, s>>>(g.x, g.sx, g.sx2, nb2, g.ldx, !g.trans_x, g.m,
-                                                                    g.k, tk, items, g.pack_x);
-    gemm_pack_kernel<MODE><<<dim3(tn * tk, by), kPThreads, 0, s>>>(g.y, g.sy, g.sy2, nb2, g.ldy, g.trans_y, g.n,
-                                                                    g.k, tk, items, g.pack_y);
+    if (!g.x_packed)
+      gemm_pack_kernel<MODE><<<dim3(tm * tk, by), kPThreads, 0, s>>>(
+          g.x, g.sx, g.sx2, nb2, g.ldx, !g.trans_x, keep_x(g.x_tri), g.m, g.k, tk, items, g.pack_x);
+    gemm_pack_kernel<MODE><<<dim3(tn * tk, by), kPThreads, 0, s>>>(
+        g.y, g.sy, g.sy2, nb2, g.ldy, g.trans_y, keep_y(g.y_tri), g.n, g.k, tk, items, g.pack_y);
     if (int st = check_launch("gemm_pack_kernel")) return st;
   }
   if (int st = ensure_smem_attr((const void*)gemm_bulk_kernel<MODE>, kGBulkSmem, slot_bulk)) return st;

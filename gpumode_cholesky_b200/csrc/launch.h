@@ -109,7 +109,7 @@ struct GemmArgs {
   int ldx, ldy, ldc;
   int m, n, k;
   int trans_x, trans_y;  // op1 = X^T / op2 = Y^T
-  int x_tri, y_tri;      // 0 none; 1: op(.) lower (op1: k <= m, op2: k >= n); 2: upper
+  int x_tri, y_tri;      // 0 none; 1: op(.) lower (op1: k <= m, op2: k >= n); 2: upper; the rest is not read
   int lower_out;         // write only C[i][j], j <= i (square M == N); skip tiles above
   int phi;               // epilogue: zero above the diagonal, halve the diagonal
   float alpha, beta;
@@ -121,6 +121,7 @@ struct GemmArgs {
   // row in every output tile.
   uint8_t* pack_x;
   uint8_t* pack_y;
+  int x_packed;          // pack_x holds op1(X) already (an earlier product's operand)
   // Optional second batch dimension (0 = none): item (b, b2) of C starts at
   // c + b sc + b2 sc2 (likewise x, y), b2 < batch2.
   int64_t batch2;

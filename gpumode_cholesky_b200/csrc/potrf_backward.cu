@@ -35,17 +35,21 @@ __global__ void __launch_bounds__(kD64Threads) trtri_diag_kernel(const float* __
   const int w = min(64, n - k0);
   for (int64_t b = blockIdx.y; b < batch; b += gridDim.y) {
     const size_t off = (size_t)b * n * n + (size_t)k0 * n + k0;
+    float* lt = diag64_lt(sm);
+#pragma unroll 8
     for (int e = tid; e < 4096; e += kD64Threads) {
       const int r = e >> 6, c = e & 63;
       float v = (r == c) ? 1.0f : 0.0f;
       if (r < w && c < w) v = (c <= r) ? l[off + (size_t)r * n + c] : 0.0f;
       sm.S[r * kD64Ld + c] = v;
+      lt[c * kD64Ld + r] = v;
     }
     __syncthreads();
     diag64_invert_only(sm);
+#pragma unroll 8
     for (int e = tid; e < 4096; e += kD64Threads) {
       const int r = e >> 6, c = e & 63;
-      if (r < w && c < w) u[off + (size_t)r * n + c] = sm.T[r * kD64Ld + c];
+      if (r < w && c < w) u[off + (size_t)r * n + c] = sm.T[c * kD64Ld + r];
     }
     __syncthreads();
   }
@@ -308,8 +312,10 @@ static GemmArgs gemm_args(int64_t batch, int n, const PackScratch& ps) {
   return g;
 }
 
-// Packing pays once both sides of a product are this large.
-constexpr int kPackMin = 256;
+// Packing pays once both sides of a product are this large: 64x256 in one
+// launch per product 200 us, packed 217; 16x500 305 and 291, 100x384 588 and
+// 557 (whole adjoint; the largest products decide).
+constexpr int kPackMin = 384;
 
 // The off-diagonal block of `pairs` block pairs ([lo, mid), [mid, hi), then
 // the same shape every 2 (mid - lo) blocks down the diagonal), each of whose
@@ -420,8 +426,8 @@ int potrf_backward(const float* l, const float* lbar, float* abar, int64_t batch
     ps.y = p0 + pack;
   }
   int32_t* err = nullptr;
-  // U = L^{-1}: zero (upper part stays zero), diagonal blocks, recursion.
-  if (cudaMemsetAsync(u, 0, mat * sizeof(float), s) != cudaSuccess) return check_launch("cudaMemsetAsync");
+  // U = L^{-1}: diagonal blocks, recursion.  Its upper part, like that of P and
+  // Z below, is neither written nor read (the products' triangular hints).
   const int nblk = (n + 63) / 64;
   if (int st = ensure_smem_attr((const void*)trtri_diag_kernel, sizeof(Diag64Smem), kSlotBwd2)) return st;
   {
@@ -433,8 +439,7 @@ int potrf_backward(const float* l, const float* lbar, float* abar, int64_t batch
   if (int st = trtri_range(l, u, w1, batch, n, nblk, 0, nblk, mode, err, ps, s)) return st;
   const PackScratch none;
   const PackScratch& pbig = n >= kPackMin ? ps : none;
-  // P = Phi(tril(L^T Lbar)) into w1 (upper part zero).
-  if (cudaMemsetAsync(w1, 0, mat * sizeof(float), s) != cudaSuccess) return check_launch("cudaMemsetAsync");
+  // P = Phi(tril(L^T Lbar)) into w1.
   GemmArgs g = gemm_args(batch, n, pbig);
   g.x = l;
   g.y = lbar;
@@ -446,8 +451,7 @@ int potrf_backward(const float* l, const float* lbar, float* abar, int64_t batch
   g.lower_out = 1;
   g.phi = 1;
   if (int st = launch_gemm_tc(g, mode, err, s)) return st;
-  // Z = P U into abar (lower; upper zero).
-  if (cudaMemsetAsync(abar, 0, mat * sizeof(float), s) != cudaSuccess) return check_launch("cudaMemsetAsync");
+  // Z = P U into abar.
   g = gemm_args(batch, n, pbig);
   g.x = w1;
   g.y = u;
@@ -457,8 +461,12 @@ int potrf_backward(const float* l, const float* lbar, float* abar, int64_t batch
   g.y_tri = 1;
   g.lower_out = 1;
   if (int st = launch_gemm_tc(g, mode, err, s)) return st;
-  // S = U^T Z into w1.
+  // S = U^T Z into w1.  U^T as the left operand is packed like U as the right
+  // one, which the product before left in its place.
   g = gemm_args(batch, n, pbig);
+  g.pack_x = pbig.y;
+  g.pack_y = pbig.x;
+  g.x_packed = pbig.x != nullptr;
   g.x = u;
   g.y = abar;
   g.c = w1;
