@@ -112,6 +112,8 @@ def lib_path() -> Path:
 def load(path: Path | None = None) -> ctypes.CDLL:
     """Load the shared object (once) and declare every exported signature."""
     global _lib
+    if _lib is not None and path is None:
+        return _lib
     with _lock:
         if _lib is not None and path is None:
             return _lib

@@ -13,10 +13,17 @@ tensor-core products.  The reference has no backward; this is an extension.
 
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from . import _lib
-from .potrf import _stream_ptr, cholesky, resolve_mode, workspace
+from .potrf import _on_device, _stream_ptr, cholesky, resolve_mode, workspace
+
+
+@functools.lru_cache(maxsize=256)
+def _workspace_size(batch: int, n: int) -> int:
+    return _lib.load().b2p_potrf_backward_workspace_size(batch, n)
 
 
 def potrf_backward(l: torch.Tensor, lbar: torch.Tensor, mode: str | int = "bf16x3") -> torch.Tensor:
@@ -33,8 +40,8 @@ def potrf_backward(l: torch.Tensor, lbar: torch.Tensor, mode: str | int = "bf16x
     code = resolve_mode(mode, n)
     abar = torch.empty_like(l)
     lib = _lib.load()
-    with torch.cuda.device(l.device):
-        ws_bytes = lib.b2p_potrf_backward_workspace_size(batch, n)
+    with _on_device(l.device):
+        ws_bytes = _workspace_size(batch, n)
         ws = workspace(l.device, ws_bytes).data_ptr() if ws_bytes else None
         st = lib.b2p_potrf_backward(
             l.data_ptr(), lbar.data_ptr(), abar.data_ptr(), batch, n, code, ws, ws_bytes, _stream_ptr(l.device)

@@ -160,7 +160,7 @@ __device__ __forceinline__ void g_mmas(uint32_t tmem, uint32_t a, uint32_t b, bo
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kGThreads, 1) gemm_tc_kernel(GemmArgs g, int tiles_n, int32_t* err) {
+__global__ void __launch_bounds__(kGThreads, 2) gemm_tc_kernel(GemmArgs g, int tiles_n, int32_t* err) {
   extern __shared__ unsigned char graw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(graw) + 1023) & ~(uintptr_t)1023);
   uint8_t* opA = base;

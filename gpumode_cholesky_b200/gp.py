@@ -17,7 +17,7 @@ import torch
 
 from . import _lib
 from .autograd import potrf_backward
-from .potrf import _stream_ptr, cholesky
+from .potrf import _on_device, _stream_ptr, cholesky
 
 
 def _check(l: torch.Tensor, v: torch.Tensor) -> None:
@@ -34,7 +34,7 @@ def trsv(l: torch.Tensor, b: torch.Tensor, trans: bool = False) -> torch.Tensor:
     _check(l, b)
     l, b = l.contiguous(), b.contiguous()
     x = torch.empty_like(b)
-    with torch.cuda.device(l.device):
+    with _on_device(l.device):
         st = _lib.load().b2p_trsv_batched(
             l.data_ptr(), b.data_ptr(), x.data_ptr(), l.shape[0], l.shape[-1], int(trans), _stream_ptr(l.device)
         )
@@ -48,7 +48,7 @@ def gp_nll_from_factor(l: torch.Tensor, y: torch.Tensor) -> tuple[torch.Tensor, 
     l, y = l.contiguous(), y.contiguous()
     alpha = torch.empty_like(y)
     loss = torch.empty(y.shape[0], dtype=torch.float32, device=y.device)
-    with torch.cuda.device(l.device):
+    with _on_device(l.device):
         st = _lib.load().b2p_gp_nll_forward(
             l.data_ptr(), y.data_ptr(), alpha.data_ptr(), loss.data_ptr(), l.shape[0], l.shape[-1],
             _stream_ptr(l.device),
@@ -63,7 +63,7 @@ def gp_nll_lbar(l: torch.Tensor, alpha: torch.Tensor, gloss: torch.Tensor) -> tu
     gloss = gloss.to(torch.float32).contiguous()
     beta = torch.empty_like(alpha)
     lbar = torch.empty_like(l)
-    with torch.cuda.device(l.device):
+    with _on_device(l.device):
         st = _lib.load().b2p_gp_nll_backward(
             l.data_ptr(), alpha.data_ptr(), gloss.data_ptr(), beta.data_ptr(), lbar.data_ptr(), l.shape[0],
             l.shape[-1], _stream_ptr(l.device),

@@ -11,15 +11,37 @@ raises, and a failing library call raises :class:`PotrfError`.
 
 from __future__ import annotations
 
+import contextlib
+import functools
+
 import torch
 
 from . import _lib
 
 _WS: dict[tuple[int, int], torch.Tensor] = {}
+_SAME_DEVICE = contextlib.nullcontext()
+
+# The smallest calls are bound by the host (a 4096x32 call's kernel takes about
+# as long as enqueueing it), so a call looks up only what it needs: the raw
+# stream handle instead of a Stream object, no device switch when the device is
+# the current one, and sizes that depend on the shape alone from a small cache.
 
 
 def _stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current stream of `device` as the integer handle the library takes."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(index if index is not None else torch.cuda.current_device())
+
+
+def _on_device(device: torch.device):
+    """Context that makes `device` current, free of cost when it is already."""
+    return _SAME_DEVICE if torch._C._cuda_getDevice() == device.index else torch.cuda.device(device)
+
+
+@functools.lru_cache(maxsize=256)
+def _workspace_size(device_index: int, batch: int, n: int, code: int, path: int) -> int:
+    """Of the current device, `device_index` (the path depends on its SM count)."""
+    return _lib.load().b2p_potrf_path_workspace_size(batch, n, code, path)
 
 
 def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
@@ -36,6 +58,7 @@ def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     return buf
 
 
+@functools.lru_cache(maxsize=256)
 def resolve_mode(mode: str | int | None, n: int) -> int:
     """Precision mode code for order n; None picks the library default (FP32).
 
@@ -107,9 +130,10 @@ def cholesky(
     elif out.shape != a.shape or out.dtype != torch.float32 or not out.is_contiguous() or out.device != a.device:
         raise ValueError("out must be a contiguous float32 tensor shaped like the input, on the same device")
     lib = _lib.load()
-    with torch.cuda.device(a.device):
-        ws_bytes = lib.b2p_potrf_path_workspace_size(batch, n, code, pcode)
-        ws_ptr = workspace(a.device, ws_bytes).data_ptr() if ws_bytes else None
+    device = a.device
+    with _on_device(device):
+        ws_bytes = _workspace_size(device.index, batch, n, code, pcode)
+        ws_ptr = workspace(device, ws_bytes).data_ptr() if ws_bytes else None
         info_ptr = None
         if info is not None:
             if info.dtype != torch.int32 or info.numel() < batch or not info.is_cuda:
@@ -122,7 +146,7 @@ def cholesky(
             from_ptr = fp32_from.data_ptr()
         st = lib.b2p_potrf_batched_ex(
             a.data_ptr(), out.data_ptr(), batch, n, code, pcode, ws_ptr, ws_bytes, info_ptr, from_ptr,
-            _stream_ptr(a.device),
+            _stream_ptr(device),
         )
     _lib.check(st, "b2p_potrf_batched_ex")
     return out

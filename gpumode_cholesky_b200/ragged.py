@@ -21,7 +21,7 @@ import torch
 
 from . import _lib
 from .inputs import pack_offsets
-from .potrf import _stream_ptr, resolve_mode
+from .potrf import _on_device, _stream_ptr, resolve_mode
 
 
 def pack(mats: Sequence[torch.Tensor], device=None) -> tuple[torch.Tensor, list[int], list[int]]:
@@ -120,7 +120,7 @@ class RaggedPlan:
             out = torch.empty_like(a)
         if info is not None and (info.dtype != torch.int32 or info.numel() < self.count):
             raise ValueError("info must be int32 with one entry per matrix")
-        with torch.cuda.device(a.device):
+        with _on_device(a.device):
             st = _lib.load().b2p_potrf_ragged(
                 self._handle,
                 self.tables.data_ptr(),
