@@ -224,6 +224,12 @@ enum SmemSlot {
   kSlotSplitW2,
   kSlotTiles,
   kSlotCta64,
+  kSlotTrsvS0,
+  kSlotTrsvS1,
+  kSlotTrsvS2,
+  kSlotTrsvS3,
+  kSlotBwdSmall64,
+  kSlotBwdSmall32,
   kSlotCount
 };
 

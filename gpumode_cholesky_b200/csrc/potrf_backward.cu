@@ -93,105 +93,84 @@ __global__ void __launch_bounds__(kSymThreads) sym_kernel(const float* __restric
 }
 
 // ---- n <= 128: one CTA per matrix ------------------------------------------
-constexpr int kBsThreads = 512;  // 16 warps: 8 x 4 register tiles over the 128 x 128 products
-constexpr int kBsLd = 132;                      // row stride of the three 128x128 buffers
-constexpr int kBsBuf = 128 * kBsLd;             // floats per buffer
-constexpr int kBsWork = 64 * 64;                // trtri128's scratch W
-constexpr size_t kBsSmemBytes = sizeof(float) * (size_t)(3 * kBsBuf + kBsWork + 128 + 4);
+// Padded to NP = 32, 64 or 128: NP^2 / 32 threads with 8 x 4 register tiles over
+// the NP x NP products, two buffers of row stride NP + 4 (L, then U in its
+// place, then S; Lbar, then P^T, then Z) and the inverse's scratch.  Padding by
+// the order keeps small matrices small: 300x24 took 134 us padded to 128 like
+// the rest, 500x40 181 us.
+template <int NP>
+struct Bs {
+  static constexpr int kThreads = NP * NP / 32;
+  static constexpr int kWarps = kThreads / 32;
+  static constexpr int kLd = NP + 4;
+  static constexpr int kWLd = NP / 2;             // scratch W: (NP / 2) x (NP / 2)
+  static constexpr int kWork = NP > 32 ? kWLd * kWLd : 0;
+  static constexpr size_t kSmem = sizeof(float) * (size_t)(2 * NP * kLd + kWork + NP);
+};
 
 // acc[r][c] = sum_{k in [k0, k1)} X[k][8ti + r] * Y[k][4tj + c] (X, Y row-major
-// in shared memory, row stride kBsLd): the X^T Y tile of this thread.
+// in shared memory, row stride LD): the X^T Y tile of this thread.
+template <int LD>
 __device__ __forceinline__ void bs_tile(const float* X, const float* Y, int ti, int tj, int k0, int k1,
                                         float (&acc)[8][4]) {
 #pragma unroll
   for (int r = 0; r < 8; ++r)
 #pragma unroll
     for (int c = 0; c < 4; ++c) acc[r][c] = 0.0f;
-#pragma unroll 2
+#pragma unroll 4
   for (int k = k0; k < k1; ++k) {
-    const float4 x0 = *reinterpret_cast<const float4*>(X + k * kBsLd + 8 * ti);
-    const float4 x1 = *reinterpret_cast<const float4*>(X + k * kBsLd + 8 * ti + 4);
-    const float4 y0 = *reinterpret_cast<const float4*>(Y + k * kBsLd + 4 * tj);
+    const float4 x0 = *reinterpret_cast<const float4*>(X + k * LD + 8 * ti);
+    const float4 x1 = *reinterpret_cast<const float4*>(X + k * LD + 8 * ti + 4);
+    const float4 y0 = *reinterpret_cast<const float4*>(Y + k * LD + 4 * tj);
     const float xv[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-    const float yv[4] = {y0.x, y0.y, y0.z, y0.w};
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(xv[r], yv[c], acc[r][c]);
+    for (int r = 0; r < 8; ++r) {
+      fma2(acc[r][0], acc[r][1], xv[r], y0.x, y0.y);
+      fma2(acc[r][2], acc[r][3], xv[r], y0.z, y0.w);
+    }
   }
 }
 
-// C = A B (NEG: -(A B)) for 64 x 64 blocks, with register tiles over the
-// 512 threads (2 rows x 4 columns each).  A and B are row-major in shared
-// memory; the K range of output column group c4 (4 columns) and row pair is
-// cut to where both operands can be non-zero: B lower triangular
-// (B[k][j] = 0 for k < j) when B_LOWER, A lower triangular (A[i][k] = 0 for
-// k > i) when A_LOWER.
-template <bool A_LOWER, bool B_LOWER, bool NEG>
-__device__ __forceinline__ void product64(const float* A, int lda, const float* B, int ldb, float* C, int ldc) {
-  const int t = threadIdx.x;
-  const int i0 = 2 * (t >> 4), j0 = 4 * (t & 15);  // rows i0, i0+1; columns j0..j0+3
-  float acc[2][4] = {};
-  const int k_lo = B_LOWER ? j0 : 0;
-  const int k_hi = A_LOWER ? i0 + 2 : 64;
-  for (int k = k_lo; k < k_hi; ++k) {
-    const float a0 = A[i0 * lda + k], a1 = A[(i0 + 1) * lda + k];
-    const float4 b = *reinterpret_cast<const float4*>(B + k * ldb + j0);
-    acc[0][0] = fmaf(a0, b.x, acc[0][0]);
-    acc[0][1] = fmaf(a0, b.y, acc[0][1]);
-    acc[0][2] = fmaf(a0, b.z, acc[0][2]);
-    acc[0][3] = fmaf(a0, b.w, acc[0][3]);
-    acc[1][0] = fmaf(a1, b.x, acc[1][0]);
-    acc[1][1] = fmaf(a1, b.y, acc[1][1]);
-    acc[1][2] = fmaf(a1, b.z, acc[1][2]);
-    acc[1][3] = fmaf(a1, b.w, acc[1][3]);
+// C = A B (NEG: -(A B)) for `count` pairs of H x H blocks: block h reads A + h
+// a_off and B + h b_off and writes C + h c_off; 1 row x 4 columns at a time.
+// A and B are row-major in shared memory; the K range is cut to where both
+// operands can be non-zero: B lower triangular (B[k][j] = 0 for k < j) when
+// B_LOWER, A lower triangular (A[i][k] = 0 for k > i) when A_LOWER.
+template <int NT, int H, bool A_LOWER, bool B_LOWER, bool NEG>
+__device__ __forceinline__ void block_product(const float* A, int lda, const float* B, int ldb, float* C, int ldc,
+                                              int count, int a_off, int b_off, int c_off) {
+  constexpr int kPer = H * H / 4;
+  for (int t = threadIdx.x; t < count * kPer; t += NT) {
+    const int h = t / kPer, u = t % kPer;
+    const int i = u / (H / 4), j0 = 4 * (u % (H / 4));
+    const float* Ah = A + h * a_off + i * lda;
+    const float* Bh = B + h * b_off + j0;
+    float acc[4] = {};
+    const int k_hi = A_LOWER ? i + 1 : H;
+#pragma unroll 4
+    for (int k = B_LOWER ? j0 : 0; k < k_hi; ++k) {
+      const float4 b = *reinterpret_cast<const float4*>(Bh + k * ldb);
+      fma2(acc[0], acc[1], Ah[k], b.x, b.y);
+      fma2(acc[2], acc[3], Ah[k], b.z, b.w);
+    }
+    const float sg = NEG ? -1.0f : 1.0f;
+    *reinterpret_cast<float4*>(C + h * c_off + i * ldc + j0) =
+        make_float4(sg * acc[0], sg * acc[1], sg * acc[2], sg * acc[3]);
   }
-  const float sg = NEG ? -1.0f : 1.0f;
-#pragma unroll
-  for (int r = 0; r < 2; ++r)
-    *reinterpret_cast<float4*>(C + (i0 + r) * ldc + j0) =
-        make_float4(sg * acc[r][0], sg * acc[r][1], sg * acc[r][2], sg * acc[r][3]);
-}
-
-// The same for two independent 32 x 32 products at once: block h = t / 256
-// reads A + h a_off and B + h b_off and writes C + h c_off; each thread
-// computes 1 row x 4 columns.
-template <bool A_LOWER, bool B_LOWER, bool NEG>
-__device__ __forceinline__ void product32x2(const float* A, int lda, const float* B, int ldb, float* C, int ldc,
-                                                int a_off, int b_off, int c_off) {
-  const int t = threadIdx.x;
-  const int h = t >> 8, u = t & 255;
-  const int i = u >> 3, j0 = 4 * (u & 7);
-  const float* Ah = A + h * a_off;
-  const float* Bh = B + h * b_off;
-  float acc[4] = {};
-  const int k_lo = B_LOWER ? j0 : 0;
-  const int k_hi = A_LOWER ? i + 1 : 32;
-  for (int k = k_lo; k < k_hi; ++k) {
-    const float a = Ah[i * lda + k];
-    const float4 b = *reinterpret_cast<const float4*>(Bh + k * ldb + j0);
-    acc[0] = fmaf(a, b.x, acc[0]);
-    acc[1] = fmaf(a, b.y, acc[1]);
-    acc[2] = fmaf(a, b.z, acc[2]);
-    acc[3] = fmaf(a, b.w, acc[3]);
-  }
-  const float sg = NEG ? -1.0f : 1.0f;
-  *reinterpret_cast<float4*>(C + h * c_off + i * ldc + j0) = make_float4(sg * acc[0], sg * acc[1], sg * acc[2], sg * acc[3]);
-}
-
-// U = L^{-1} of the 128 x 128 lower-triangular L in shared memory (row stride
-// ld), into U (row stride ld, zero above the diagonal), by block recursion:
-//   32 x 32 diagonal blocks by forward substitution (warp b, lane = column);
-//   U_10 = -U_11 (L_10 U_00) inside each 64-block (both 64-blocks at once);
-//   U_21 = -U_22 (L_21 U_11) for the 64-blocks.
-// invd holds 1 / L_ii; W is scratch of 64 x kBsWLd floats.  All 512 threads.
-constexpr int kBsWLd = 64;
-static_assert(64 * kBsWLd <= kBsWork, "trtri128 scratch fits the work area");
-__device__ void trtri128(const float* L, float* U, int ld, const float* invd, float* W) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int e = tid; e < 128 * ld; e += kBsThreads) U[e] = 0.0f;
   __syncthreads();
-  if (warp < 4) {
+}
+
+// U = L^{-1} of the NP x NP lower-triangular L in shared memory, in place
+// (zero above the diagonal before and after), by block recursion:
+//   32 x 32 diagonal blocks by forward substitution (warp b, lane = column);
+//   U_10 = -U_11 (L_10 U_00) for the 32-blocks of each 64-block, then for the
+//   64-blocks.
+// invd holds 1 / L_ii; W is scratch.
+template <int NP>
+__device__ void trtri_small(float* L, const float* invd, float* W) {
+  constexpr int kLd = Bs<NP>::kLd, kNT = Bs<NP>::kThreads;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (warp < NP / 32) {
     const int kb = 32 * warp, c = lane;
     float x[32];
 #pragma unroll
@@ -200,57 +179,60 @@ __device__ void trtri128(const float* L, float* U, int ld, const float* invd, fl
     for (int m = 0; m < 32; ++m) {
       x[m] *= invd[kb + m];
 #pragma unroll
-      for (int j = m + 1; j < 32; ++j) x[j] = fmaf(-L[(kb + j) * ld + kb + m], x[m], x[j]);
+      for (int j = m + 1; j < 32; ++j) x[j] = fmaf(-L[(kb + j) * kLd + kb + m], x[m], x[j]);
     }
+    __syncwarp();
 #pragma unroll
     for (int j = 0; j < 32; ++j)
-      if (j >= c) U[(kb + j) * ld + kb + c] = x[j];
+      if (j >= c) L[(kb + j) * kLd + kb + c] = x[j];
   }
   __syncthreads();
-  // Inside each 64-block h: W_h = L_10 U_00 (W rows 32 h ..), then U_10 = -U_11 W_h.
-  // Block h covers rows / columns 64 h .. 64 h + 63; its L_10 starts at
-  // (64 h + 32, 64 h), U_00 at (64 h, 64 h), U_11 at (64 h + 32, 64 h + 32).
-  product32x2<false, true, false>(L + 32 * ld, ld, U, ld, W, kBsWLd, 64 * (ld + 1), 64 * (ld + 1), 32 * kBsWLd);
-  __syncthreads();
-  product32x2<true, false, true>(U + 32 * ld + 32, ld, W, kBsWLd, U + 32 * ld, ld, 64 * (ld + 1), 32 * kBsWLd,
-                                 64 * (ld + 1));
-  __syncthreads();
-  // W = L_21 U_11 (the first 64-block's inverse), then U_21 = -U_22 W.
-  product64<false, true, false>(L + 64 * ld, ld, U, ld, W, kBsWLd);
-  __syncthreads();
-  product64<true, false, true>(U + 64 * ld + 64, ld, W, kBsWLd, U + 64 * ld, ld);
-  __syncthreads();
+  if (NP >= 64) {
+    constexpr int kPairs = NP / 64, kStep = 64 * (kLd + 1);
+    block_product<kNT, 32, false, true, false>(L + 32 * kLd, kLd, L, kLd, W, 32, kPairs, kStep, kStep, 32 * 32);
+    block_product<kNT, 32, true, false, true>(L + 32 * kLd + 32, kLd, W, 32, L + 32 * kLd, kLd, kPairs, kStep,
+                                              32 * 32, kStep);
+  }
+  if (NP == 128) {
+    block_product<kNT, 64, false, true, false>(L + 64 * kLd, kLd, L, kLd, W, 64, 1, 0, 0, 0);
+    block_product<kNT, 64, true, false, true>(L + 64 * kLd + 64, kLd, W, 64, L + 64 * kLd, kLd, 1, 0, 0, 0);
+  }
 }
 
-__global__ void __launch_bounds__(kBsThreads, 1)
+template <int NP>
+__global__ void __launch_bounds__(Bs<NP>::kThreads)
     bwd_small_kernel(const float* __restrict__ l, const float* __restrict__ lbar, float* __restrict__ abar,
                      int64_t batch, int n) {
   extern __shared__ __align__(16) float bsm[];
-  float* bA = bsm;               // L, later S
-  float* bB = bsm + kBsBuf;      // Lbar, later P^T, later Z
-  float* bC = bsm + 2 * kBsBuf;  // U = L^{-1}
-  float* work = bsm + 3 * kBsBuf;
-  float* invd = work + kBsWork;
-  const int tid = threadIdx.x;
-  const int ti = tid >> 5, tj = tid & 31;  // rows 8ti.., columns 4tj..
+  constexpr int kLd = Bs<NP>::kLd;
+  float* bA = bsm;                       // L, U, S
+  float* bB = bsm + NP * kLd;            // Lbar, P^T, Z
+  float* work = bsm + 2 * NP * kLd;
+  float* invd = work + Bs<NP>::kWork;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ti = tid / (NP / 4), tj = tid % (NP / 4);  // rows 8ti.., columns 4tj..
   float acc[8][4];
   for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
     const float* L = l + (size_t)b * n * n;
     const float* G = lbar + (size_t)b * n * n;
     // L (lower, identity beyond n) and Lbar (lower, zero beyond n).
-    for (int e = tid; e < 128 * 128; e += kBsThreads) {
-      const int i = e >> 7, j = e & 127;
-      const bool in = i < n && j < n && j <= i;
-      bA[i * kBsLd + j] = in ? L[(size_t)i * n + j] : (i == j ? 1.0f : 0.0f);
-      bB[i * kBsLd + j] = in ? G[(size_t)i * n + j] : 0.0f;
-    }
+#pragma unroll 4
+    for (int i = warp; i < NP; i += Bs<NP>::kWarps)
+#pragma unroll
+      for (int j0 = 0; j0 < NP; j0 += 32) {
+        const int j = j0 + lane;
+        const bool in = i < n && j <= i;
+        bA[i * kLd + j] = in ? L[(size_t)i * n + j] : (i == j ? 1.0f : 0.0f);
+        bB[i * kLd + j] = in ? G[(size_t)i * n + j] : 0.0f;
+      }
     __syncthreads();
-    if (tid < 128) invd[tid] = 1.0f / bA[tid * kBsLd + tid];
+    if (tid < NP) invd[tid] = 1.0f / bA[tid * kLd + tid];
+    if (Bs<NP>::kThreads < NP) __syncthreads();
     // P = Phi(L^T Lbar) (tiles reaching the lower triangle; k >= max(i, j)),
     // kept in registers.
     const bool lower = 4 * tj <= 8 * ti + 7;
     const int kmax = 8 * ti > 4 * tj ? 8 * ti : 4 * tj;  // smallest max(i, j) of the tile
-    if (lower) bs_tile(bA, bB, ti, tj, kmax, 128, acc);
+    if (lower) bs_tile<kLd>(bA, bB, ti, tj, kmax, NP, acc);
     __syncthreads();
     // P^T into bB: per column j of the tile, its 8 rows as two float4.
 #pragma unroll
@@ -262,35 +244,47 @@ __global__ void __launch_bounds__(kBsThreads, 1)
         const int i = 8 * ti + r;
         v[r] = !lower || j > i ? 0.0f : (j == i ? 0.5f * acc[r][c] : acc[r][c]);
       }
-      float4* dst = reinterpret_cast<float4*>(bB + j * kBsLd + 8 * ti);
+      float4* dst = reinterpret_cast<float4*>(bB + j * kLd + 8 * ti);
       dst[0] = make_float4(v[0], v[1], v[2], v[3]);
       dst[1] = make_float4(v[4], v[5], v[6], v[7]);
     }
-    // U = L^{-1} into bC.
-    trtri128(bA, bC, kBsLd, invd, work);
+    // U = L^{-1} in L's place.
+    trtri_small<NP>(bA, invd, work);
     // Z = P U: Z[i][j] = sum_k P^T[k][i] U[k][j], k in [j, i] (lower tiles).
-    if (lower) bs_tile(bB, bC, ti, tj, 4 * tj, 8 * ti + 8, acc);
+    if (lower) bs_tile<kLd>(bB, bA, ti, tj, 4 * tj, 8 * ti + 8, acc);
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
       const int i = 8 * ti + r, j = 4 * tj;
-      *reinterpret_cast<float4*>(bB + i * kBsLd + j) =
+      *reinterpret_cast<float4*>(bB + i * kLd + j) =
           make_float4((lower && j <= i) ? acc[r][0] : 0.0f, (lower && j + 1 <= i) ? acc[r][1] : 0.0f,
                       (lower && j + 2 <= i) ? acc[r][2] : 0.0f, (lower && j + 3 <= i) ? acc[r][3] : 0.0f);
     }
     __syncthreads();
     // S = U^T Z: S[i][j] = sum_k U[k][i] Z[k][j], k >= max(i, j); into bA.
-    bs_tile(bC, bB, ti, tj, kmax, 128, acc);
+    bs_tile<kLd>(bA, bB, ti, tj, kmax, NP, acc);
+    __syncthreads();
 #pragma unroll
     for (int r = 0; r < 8; ++r)
-      *reinterpret_cast<float4*>(bA + (8 * ti + r) * kBsLd + 4 * tj) =
+      *reinterpret_cast<float4*>(bA + (8 * ti + r) * kLd + 4 * tj) =
           make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
     __syncthreads();
     float* Ab = abar + (size_t)b * n * n;
-    for (int i = tid >> 5; i < n; i += kBsThreads / 32)
-      for (int j = tid & 31; j < n; j += 32) Ab[(size_t)i * n + j] = 0.5f * (bA[i * kBsLd + j] + bA[j * kBsLd + i]);
+    for (int i = warp; i < n; i += Bs<NP>::kWarps)
+#pragma unroll 4
+      for (int j = lane; j < n; j += 32) Ab[(size_t)i * n + j] = 0.5f * (bA[i * kLd + j] + bA[j * kLd + i]);
     __syncthreads();
   }
+}
+
+template <int NP>
+static int launch_bwd_small(const float* l, const float* lbar, float* abar, int64_t batch, int n, int slot,
+                            cudaStream_t s) {
+  if (int st = ensure_smem_attr((const void*)bwd_small_kernel<NP>, Bs<NP>::kSmem, slot)) return st;
+  TraceScope ts(kKBwdSym, s);
+  const int grid = (int)std::min<int64_t>(batch, (int64_t)device_sms() * (NP == 128 ? 1 : 16));
+  bwd_small_kernel<NP><<<grid, Bs<NP>::kThreads, Bs<NP>::kSmem, s>>>(l, lbar, abar, batch, n);
+  return check_launch("bwd_small_kernel");
 }
 
 // Packed-operand scratch of the current call (see GemmArgs::pack_x).
@@ -406,11 +400,9 @@ int potrf_backward(const float* l, const float* lbar, float* abar, int64_t batch
     return set_error(B2P_ERR_UNSUPPORTED, "backward runs its products in tf32 or bf16x3 (mode 0x%x)", mode);
   if (n <= 128) {
     // One CTA per matrix, everything in shared memory, FP32 in every mode.
-    if (int st = ensure_smem_attr((const void*)bwd_small_kernel, kBsSmemBytes, kSlotBwdSmall)) return st;
-    TraceScope ts(kKBwdSym, s);
-    const int grid = (int)std::min<int64_t>(batch, (int64_t)device_sms());
-    bwd_small_kernel<<<grid, kBsThreads, kBsSmemBytes, s>>>(l, lbar, abar, batch, n);
-    return check_launch("bwd_small_kernel");
+    if (n <= 32) return launch_bwd_small<32>(l, lbar, abar, batch, n, kSlotBwdSmall32, s);
+    if (n <= 64) return launch_bwd_small<64>(l, lbar, abar, batch, n, kSlotBwdSmall64, s);
+    return launch_bwd_small<128>(l, lbar, abar, batch, n, kSlotBwdSmall, s);
   }
   const size_t need = backward_workspace_bytes(batch, n);
   if (ws == nullptr || ws_bytes < need)

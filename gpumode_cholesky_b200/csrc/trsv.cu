@@ -18,6 +18,10 @@
 // its own remaining rows (one row per thread and 32 loads in flight for L,
 // float4 column groups for L^T).  All FP32.
 //
+// Orders up to 128 take trsv_small_kernel instead: the factor in shared memory,
+// thread i on row (or column) i, in short loops; for the GP backward it also
+// writes Lbar.
+//
 // The reference has no GP path (its task is the forward factorization
 // only); these implement the GP-solve step of its roadmap, with torch's
 // solve_triangular and autograd in FP64 as the oracle.
@@ -447,6 +451,142 @@ __global__ void __launch_bounds__(kTrsvThreads, 2) trsv_kernel(const float* __re
   }
 }
 
+// ---- n <= 128: one small CTA per matrix -----------------------------------------
+// Latency is all there is here: 8x33 took 16.7 us in the kernel above, most of
+// it fetching its unrolled code and its operands a step at a time.  So the
+// whole lower triangle is copied to shared memory at once, and the loops stay
+// loops.  Thread i has row i of L (column i for L^T); warp k solves diagonal
+// block k with one shuffle per pivot, and the others subtract its 32 solved
+// values.  Same values as above for L; L^T sums a block's 32 products in order.
+// Device us before and now: 256x128 GP forward 31 -> 12, solve with L^T and
+// Lbar 42 -> 19 (one launch of two); per call in a graph 16x100 28 -> 10 and
+// 27 -> 16, 8x33 16.7 -> 7.1.
+constexpr int kSmallMaxN = 128;
+enum SmallOut { kOutX = 0, kOutLoss = 1, kOutLbar = 2 };
+
+inline int small_ld(int n) { return ((n + 3) & ~3) + 4; }
+
+template <bool TRANS, int OUT>
+__global__ void __launch_bounds__(kSmallMaxN) trsv_small_kernel(const float* __restrict__ l, const float* b,
+                                                                float* xout, float* __restrict__ loss,
+                                                                const float* __restrict__ gloss,
+                                                                float* __restrict__ lbar, int64_t batch, int n) {
+  extern __shared__ __align__(16) float ss[];  // L, row stride ld
+  __shared__ float xs[kSmallMaxN], bs[kSmallMaxN], red[2][4];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+  const int ld = ((n + 3) & ~3) + 4;
+  const int nb = (n + 31) / 32;
+  const bool vec = (n & 3) == 0 && (reinterpret_cast<uintptr_t>(l) & 15u) == 0;
+  const int i = tid, ic = min(i, n - 1);
+  for (int64_t m = blockIdx.x; m < batch; m += gridDim.x) {
+    const float* L = l + (size_t)m * n * n;
+#pragma unroll 4
+    for (int r = warp; r < n; r += warps) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(ss + r * ld);
+      if (vec) {
+        if (4 * lane <= r)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * lane),
+                       "l"(L + (size_t)r * n + 4 * lane)
+                       : "memory");
+      } else {
+        for (int c = lane; c <= r; c += 32)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4 * c), "l"(L + (size_t)r * n + c)
+                       : "memory");
+      }
+    }
+    float r = i < n ? b[(size_t)m * n + i] : 0.0f;
+    if (OUT == kOutLbar) bs[i] = r;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const float inv = i < n ? 1.0f / ss[ic * (ld + 1)] : 0.0f;
+#pragma unroll 1
+    for (int s = 0; s < nb; ++s) {
+      const int blk = TRANS ? nb - 1 - s : s;
+      const int r0 = 32 * blk, w = min(32, n - r0);
+      if (warp == blk) {
+#pragma unroll 4
+        for (int jj = 0; jj < w; ++jj) {
+          const int j = TRANS ? w - 1 - jj : jj;
+          const float e = TRANS ? ss[(r0 + j) * ld + ic] : ss[ic * ld + r0 + j];
+          const float xj = __shfl_sync(0xffffffffu, r * inv, j);
+          if (lane == j) r = xj;
+          if (TRANS ? lane < j : lane > j) r = fmaf(-e, xj, r);
+        }
+        xs[i] = r;
+      }
+      __syncthreads();
+      if (TRANS ? i < r0 : (i >= r0 + 32 && i < n)) {
+        float acc = 0.0f;
+        if (TRANS) {
+#pragma unroll 8
+          for (int j = 0; j < w; ++j) acc = fmaf(ss[(r0 + j) * ld + i], xs[r0 + j], acc);
+        } else {
+#pragma unroll 2
+          for (int j = 0; j < 32; j += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(ss + i * ld + r0 + j);
+            acc = fmaf(v.x, xs[r0 + j], acc);
+            acc = fmaf(v.y, xs[r0 + j + 1], acc);
+            acc = fmaf(v.z, xs[r0 + j + 2], acc);
+            acc = fmaf(v.w, xs[r0 + j + 3], acc);
+          }
+        }
+        r -= acc;
+      }
+    }
+    if (i < n) xout[(size_t)m * n + i] = r;
+    if (OUT == kOutLoss) {
+      float quad = i < n ? r * r : 0.0f, logdet = i < n ? logf(ss[ic * (ld + 1)]) : 0.0f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        quad += __shfl_xor_sync(0xffffffffu, quad, o);
+        logdet += __shfl_xor_sync(0xffffffffu, logdet, o);
+      }
+      if (lane == 0) {
+        red[0][warp] = quad;
+        red[1][warp] = logdet;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        float t[2];
+        for (int q = 0; q < 2; ++q) {
+          float v[4];
+          for (int k = 0; k < 4; ++k) v[k] = k < warps ? red[q][k] : 0.0f;
+          t[q] = (v[0] + v[2]) + (v[1] + v[3]);
+        }
+        loss[m] = 0.5f * t[0] + t[1];
+      }
+    }
+    if (OUT == kOutLbar) {
+      // Row i of Lbar from beta_i (xs), alpha (bs) and L_ii.
+      const float g = __ldg(gloss + m);
+      float* out = lbar + (size_t)m * n * n;
+      __syncthreads();
+      for (int row = warp; row < n; row += warps) {
+        const float bi = g * xs[row];
+        const float dinv = g / ss[row * (ld + 1)];
+#pragma unroll 4
+        for (int j = lane; j < n; j += 32) {
+          const float v = -bi * bs[j];
+          out[(size_t)row * n + j] = j > row ? 0.0f : (j == row ? v + dinv : v);
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <bool TRANS, int OUT>
+int launch_small(const float* l, const float* b, float* x, float* loss, const float* gloss, float* lbar,
+                 int64_t batch, int n, int slot, int kid, cudaStream_t s) {
+  const size_t smem = (size_t)n * small_ld(n) * sizeof(float);
+  auto kern = trsv_small_kernel<TRANS, OUT>;
+  if (int st = ensure_smem_attr((const void*)kern, smem, slot)) return st;
+  const int grid = (int)std::min<int64_t>(batch, (int64_t)device_sms() * 32);
+  TraceScope ts(kid, s);
+  kern<<<grid, 32 * ((n + 31) / 32), smem, s>>>(l, b, x, loss, gloss, lbar, batch, n);
+  return check_launch("trsv_small_kernel");
+}
+
 // Lbar, one warp per row (matrix, i); float4 stores when n % 4 == 0.
 __global__ void __launch_bounds__(kTrsvThreads) gp_lbar_kernel(const float* __restrict__ l,
                                                                const float* __restrict__ alpha,
@@ -527,6 +667,9 @@ int launch_trsv_kernel(const float* l, const float* b, float* x, float* loss, in
 }  // namespace
 
 int launch_trsv(const float* l, const float* b, float* x, int64_t batch, int n, bool trans, cudaStream_t s) {
+  if (n <= kSmallMaxN)
+    return trans ? launch_small<true, kOutX>(l, b, x, nullptr, nullptr, nullptr, batch, n, kSlotTrsvS1, kKTrsv, s)
+                 : launch_small<false, kOutX>(l, b, x, nullptr, nullptr, nullptr, batch, n, kSlotTrsvS0, kKTrsv, s);
   if (trans) return launch_trsv_kernel<true, false>(l, b, x, nullptr, batch, n, kSlotTrsv1, kKTrsv, "trsv_kernel", s);
   return launch_trsv_kernel<false, false>(l, b, x, nullptr, batch, n, kSlotTrsv0, kKTrsv, "trsv_kernel", s);
 }
@@ -553,6 +696,8 @@ int b2p_gp_nll_forward(const float* l, const float* y, float* alpha, float* loss
     const cudaError_t e = cudaMemsetAsync(loss, 0, (size_t)batch * sizeof(float), s);
     return e == cudaSuccess ? B2P_OK : set_error(B2P_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
   }
+  if (n <= kSmallMaxN)
+    return launch_small<false, kOutLoss>(l, y, alpha, loss, nullptr, nullptr, batch, (int)n, kSlotTrsvS2, kKGpForward, s);
   return launch_trsv_kernel<false, true>(l, y, alpha, loss, batch, (int)n, kSlotGpForward, kKGpForward,
                                          "gp_forward_kernel", s);
 }
@@ -564,6 +709,8 @@ int b2p_gp_nll_backward(const float* l, const float* alpha, const float* gloss, 
     return set_error(B2P_ERR_INVALID_ARG, "null pointer");
   if (batch == 0 || n == 0) return B2P_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (n <= kSmallMaxN)
+    return launch_small<true, kOutLbar>(l, alpha, beta, nullptr, gloss, lbar, batch, (int)n, kSlotTrsvS3, kKGpLbar, s);
   if (int st = launch_trsv(l, alpha, beta, batch, (int)n, true, s)) return st;
   const int64_t rows = batch * n;
   const int64_t per_cta = kTrsvThreads / 32;
