@@ -13,28 +13,26 @@
 
 namespace b2p {
 
-// Row stride of transposed 32x32 copies.
-constexpr int kLtLd = 36;
-
 // Factor the 32x32 block x[] (row `lane`), columns >= w / rows >= w are
 // identity padding.  On return x holds L (lower part valid, upper part is
-// don't-care) and inv_pivot holds 1/L[lane][lane].  Returns the first local
-// pivot index that was not positive, or -1.  All 32 lanes must call.
+// don't-care).  NORMAL (see rsqrt_refined): returns 0, or a non-zero value if
+// a pivot was not a normal positive number, and the caller starts again with
+// the general form; that returns the first local pivot index that was not
+// positive, or -1.  All 32 lanes must call.
 //
 // Step k takes the pivot d = x[k] of lane k and, in the same round of
 // shuffles, lane k+1's unscaled column-k value e; every lane then forms
 // L[k+1][k] = e / sqrt(d) itself and updates its column k+1 at once, so the
 // next pivot depends only on shuffles and registers.  The rest of the rank-1
 // update (columns k+2..31) goes through a double-buffered shared-memory copy
-// of column k and is deferred by one step: step k+1 applies it right after
-// shuffling out its own pivot, in the shadow of that pivot's reciprocal
-// square root.  The arithmetic is the same as the textbook right-looking
-// update, value for value and in the same order.
-__device__ __forceinline__ int warp_factor32(float (&x)[32], int lane, int w, float* colbuf,
-                                             float& inv_pivot) {
-  int bad = -1;
-  inv_pivot = 1.0f;
-  float lprev = 0.0f;  // this lane's L[lane][k-1]
+// of column k and is deferred by one step: step k+1 applies it, two columns an
+// instruction, right after shuffling out its own pivot, in the shadow of that
+// pivot's reciprocal square root.  The arithmetic is the same as the textbook
+// right-looking update, value for value and in the same order.
+template <bool NORMAL>
+__device__ __forceinline__ int warp_factor32(float (&x)[32], int lane, int w, float* colbuf) {
+  int bad = NORMAL ? 0 : -1;
+  float nlprev = 0.0f;  // minus this lane's L[lane][k-1]
 #pragma unroll
   for (int k = 0; k < 32; ++k) {
     if (k < w) {  // warp-uniform
@@ -48,18 +46,23 @@ __device__ __forceinline__ int warp_factor32(float (&x)[32], int lane, int w, fl
           const float4 c = reinterpret_cast<const float4*>(cb)[j4];
           const float cv[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
+          for (int q = 0; q < 4; q += 2) {
             const int j = 4 * j4 + q;
-            if (j > k) x[j] = fmaf(-lprev, cv[q], x[j]);
+            if (j > k)
+              fma2(x[j], x[j + 1], nlprev, cv[q], cv[q + 1]);
+            else if (j + 1 > k)
+              x[j + 1] = fmaf(nlprev, cv[q + 1], x[j + 1]);
           }
         }
       }
-      if (bad < 0 && pivot_bad(d)) bad = k;
-      const float y = rsqrt_refined(d);
-      if (lane == k) inv_pivot = y;
+      if (NORMAL)
+        bad |= pivot_normal(d) ? 0 : 1;
+      else if (bad < 0 && pivot_bad(d))
+        bad = k;
+      const float y = rsqrt_refined<NORMAL>(d);
       x[k] = (lane == k) ? d * y : x[k] * y;
-      if (k + 1 < 32) x[k + 1] = fmaf(-x[k], e * y, x[k + 1]);
-      lprev = x[k];
+      nlprev = -x[k];
+      if (k + 1 < 32) x[k + 1] = fmaf(nlprev, e * y, x[k + 1]);
       if (k + 2 < 32) {
         colbuf[(k & 1) * 32 + lane] = x[k];
         __syncwarp();
