@@ -27,11 +27,11 @@
 //       and the panel copy of X.  CTA 0 of the matrix writes L_kk and info;
 //       the zero strip right of the diagonal block goes out as bulk stores.
 //
-//   split_wide_kernel       (n >= kWideMinN) the panels older than the
-//       previous 512-column outer block, applied to a whole outer block at
-//       once as 128 x 256 tensor-core tiles on a third stream, so that the
-//       per-column look-ahead only applies the last 8-15 panels (see the
-//       schedule above potrf_split).
+//   split_wide_kernel       (enough block rows, wide_width) the panels older
+//       than the previous outer block of W block columns, applied to a whole
+//       outer block at once as 128 x 256 tensor-core tiles on a third stream,
+//       so that the per-column look-ahead only applies the last W to 2W - 1
+//       panels (see the schedule above potrf_split).
 //
 // A is read once and L written once; the panel copies (4 bytes per element
 // in either mode) are the only re-read data and mostly hit L2.  Results are
@@ -220,8 +220,8 @@ __global__ void __launch_bounds__(kUThreads, 2)
 }
 
 // ---- wide update kernel ----------------------------------------------------------
-// For large orders the panels older than the previous outer block (kWideCols
-// block columns) are applied to a whole outer block at once:
+// With outer blocks (wide_width) the panels older than the previous one
+// are applied to a whole outer block at once:
 //   Out[r, j] = base[r, j] - sum_{c in [c_begin, c_end)} L_c[r] L_c[j0 + j]^T,
 //   rows r >= j0, columns j < nbw,
 // as 128 x 256 tiles (MMA N = 256: each A tile of the panel copies feeds 256
@@ -491,14 +491,13 @@ constexpr uint32_t kSZeroBytes = 4096;
 constexpr uint32_t kSDiag = kSZero + kSZeroBytes;
 constexpr uint32_t kSBar = kSDiag + (((uint32_t)sizeof(Diag64Smem) + 127u) & ~127u);
 constexpr uint32_t kSSmemBytes = kSBar + 64 + 1024;
-// Beside the outer-block update (n >= kWideMinN) two step CTAs share an SM
-// (shared memory and 2 x 128 TMEM columns), so a column's chunks need half
-// as many of the SMs it leaves free.  Below that the steps have the whole
-// GPU, and a larger request keeps each step CTA alone on its SM (neither a
-// second step CTA nor a look-ahead update CTA fits beside it): 1 x 8192 ran
-// 3286 us that way and 3769 us with the SMs shared.
+// Two step CTAs share an SM, also with look-ahead update CTAs (shared memory and
+// TMEM columns): a column's chunks need half as many SMs, and the update, which
+// has more work the larger the order, finds room beside them.  One step CTA per
+// SM (by a larger request) / two, us: 1x2048 650 / 651, 8x2048 971 / 812, 1x4096
+// 1407 / 1314, 1x8192 3721 / 3369, 20x1280 694 / 591, 8x1536 506 or 656 (from
+// process to process) / 538.
 static_assert(2 * (kSSmemBytes + 1024) <= 228 * 1024, "two step CTAs per SM");
-constexpr uint32_t kSSmemAlone = 140 * 1024;
 constexpr uint32_t kSTmemCols = 128;   // [0, 64): diagonal rows; [64, 128): the CTA's rows
 
 // Column k of every matrix, G CTAs per matrix.  P = base - X_{k-1} X_{k-1,kk}^T
@@ -757,19 +756,29 @@ __global__ void fp8_scale_kernel(const float* __restrict__ a, float* __restrict_
   sig[id] = (v > 0.0f && isfinite(v)) ? exp2f(ceilf(log2f(v))) : 1.0f;
 }
 
-// Orders from which the older panels are applied an outer block at a time
-// (split_wide_kernel), and the outer block width in block columns.  At
-// 1 x 8192 the wide stage does not pay yet (3681 us against 3628 us).
-constexpr int kWideMinN = 12288;
-constexpr int kWideCols = 8;  // 512 columns
-static_assert(64 * kWideCols % kXCols == 0, "outer blocks are whole wide tiles");
+// The width, in block columns, of the outer blocks that the older panels are
+// applied to at a time (split_wide_kernel), or 0 for none.  Without it every
+// column reads all earlier panels of 128 x 64 tiles, 48 KB per 2^19
+// multiply-adds, and from some 100 block rows of matrices on that outlasts the
+// step it hides behind (1 x 8192: the middle steps waited 6 us each).  Measured
+// on B200 with two step CTAs per SM, us, none / 4 / 8: 1x4096 1314 / 1367 /
+// 1335, 2x3072 1036 / 1046 / 1030, 1x6144 2151 / 2136 / 2123, 1x7168 2615 /
+// 2466 / 2482, 1x8192 3369 / 2858 / 2924, 1x10240 5424 / 3994 / 4007, 4x3072
+// 1163 / 1107 / 1152, 8x2048 812 / 761 / 804, 16x1536 717 / 685 / 724.
+constexpr int kWideMinRows = 104;   // batch x block rows
+constexpr int kWideLargeN = 12288;  // 8 from here (1 x 16384: 8 best of 4, 8, 16)
+static_assert(64 * 4 % kXCols == 0, "outer blocks are whole wide tiles");
+static int wide_width(int64_t batch, int64_t n) {
+  if (n >= kWideLargeN) return 8;
+  return batch * (n / 64) >= kWideMinRows ? 4 : 0;
+}
 
 // Panel copies, then two per-matrix FP32 panel buffers (n x 64 each; block
-// columns alternate between them), then for large orders two per-matrix
-// outer-block buffers (n x 512 each, alternating by outer block).
+// columns alternate between them), then with outer blocks two per-matrix
+// outer-block buffers (n x 64 wide_width each, alternating by outer block).
 static size_t split_sig_offset(int64_t batch, int64_t n) {
   size_t bytes = (size_t)batch * 2 * panel_copy_region_bytes((int)n) + 2 * (size_t)batch * n * 64 * sizeof(float);
-  if (n >= kWideMinN) bytes += 2 * (size_t)batch * n * 64 * kWideCols * sizeof(float);
+  bytes += 2 * (size_t)batch * n * 64 * wide_width(batch, n) * sizeof(float);
   return bytes;
 }
 size_t split_workspace_bytes(int64_t batch, int64_t n) {
@@ -829,8 +838,8 @@ int side_stream(SideStream** out) {
 // step(j) waits for look-ahead(j) (join event j % 2).  Column j uses panel
 // buffer j % 2, which look-ahead(j+2) may only overwrite after step(j).
 //
-// Large orders (n >= kWideMinN) split the look-ahead further.  With outer
-// blocks of W = kWideCols block columns, the panels older than the previous
+// With outer blocks the look-ahead is split further.  With outer
+// blocks of W = wide_width block columns, the panels older than the previous
 // outer block are final a whole outer block before they are needed: right
 // after the last step of outer block J-2, the wide stream computes
 //   Bw_J = A[:, block J] - (panels 0 .. (J-1) W - 1) applied to block J
@@ -865,7 +874,7 @@ int potrf_split(const float* a, float* l, int64_t batch, int n, int mode, void* 
   const int sslot[3] = {kSlotSplitS0, kSlotSplitS1, kSlotSplitS2};
   const int wslot[3] = {kSlotSplitW0, kSlotSplitW1, kSlotSplitW2};
   if (int st = ensure_smem_attr((const void*)upd, kUSmemBytes, uslot[mi])) return st;
-  if (int st = ensure_smem_attr((const void*)stp, kSSmemAlone, sslot[mi])) return st;
+  if (int st = ensure_smem_attr((const void*)stp, kSSmemBytes, sslot[mi])) return st;
   float* sig = reinterpret_cast<float*>(copies + split_sig_offset(batch, n));
   if (m == B2P_MODE_FP8) {
     const int64_t blocks = batch * (n / 64);
@@ -874,8 +883,8 @@ int potrf_split(const float* a, float* l, int64_t batch, int n, int mode, void* 
   }
   const int N = n / 64;
   const int64_t n2 = (int64_t)n * n;
-  const bool wide = n >= kWideMinN;
-  constexpr int W = kWideCols;
+  const int W = std::max(1, wide_width(batch, n));
+  const bool wide = wide_width(batch, n) > 0;
   const int nbw = 64 * W;
   float* bw[2] = {nullptr, nullptr};
   if (wide) {
@@ -947,10 +956,8 @@ int potrf_split(const float* a, float* l, int64_t batch, int n, int mode, void* 
     if (e != cudaSuccess) return set_error(B2P_ERR_CUDA, "split_wide_kernel: %s", cudaGetErrorString(e));
     return B2P_OK;
   };
-  // Step CTAs of column k: two per SM on the SMs the wide kernel leaves
-  // free, else one per SM.
-  const int64_t step_sms = wide ? 2 * (sms - wide_ctas) : sms;
-  const uint32_t step_smem = wide ? kSSmemBytes : kSSmemAlone;
+  // Step CTAs of column k: two per SM, on the SMs the wide kernel leaves free.
+  const int64_t step_sms = 2 * (wide ? sms - wide_ctas : sms);
   auto step_G = [&](int k) -> int {
     const int chunks = (n - 64 * k - 64 + kSThreads - 1) / kSThreads;
     return (int)std::max<int64_t>(1, std::min<int64_t>(std::max(chunks, 1), step_sms / batch));
@@ -977,7 +984,7 @@ int potrf_split(const float* a, float* l, int64_t batch, int n, int mode, void* 
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)grid, 1, 1);
       cfg.blockDim = dim3(kSThreads, 1, 1);
-      cfg.dynamicSmemBytes = step_smem;
+      cfg.dynamicSmemBytes = kSSmemBytes;
       cfg.stream = s;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributePriority;
