@@ -193,6 +193,9 @@ __device__ __forceinline__ void subst16(float (&x)[16], const float* lt, const f
 // is the same on every lane.
 template <bool NORMAL>
 __device__ __forceinline__ int factor16(float (&x)[16], int lane, float* invd) {
+  // A warp whose lanes come here apart (after a branch on the thread index)
+  // would meet at every shuffle anew, at 30 times the cost.
+  __syncwarp();
   int bad = NORMAL ? 0 : -1;
   float lp[4] = {0.f, 0.f, 0.f, 0.f};  // this lane's L of the previous group
 #pragma unroll
