@@ -298,19 +298,23 @@ __global__ void __launch_bounds__(kFThreads, 2)
           __syncthreads();
         }
         // X = P T^T for the rows below the diagonal block (triangle skipped),
-        // then L and the tensor-core copy from X^T.
-        xgemm_tri_inplace(PtT, kFPtLd, dg.T, kD64Ld, CtaBarrier());
-        for (int item = tid; item < kFM * 8; item += kFThreads) {
-          const int rl = item & (kFM - 1), c = item >> 7;
-          if (rl >= vr || (mt == 0 && rl < 64)) continue;
-          float v[8];
+        // then L and the tensor-core copy, lines at a time.
+        xgemm_tri(PtT, kFPtLd, dg.T, kD64Ld, CtaBarrier());
+        const int first = mt == 0 ? 64 : 0;  // rows above are the diagonal block's
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = PtT[(8 * c + j) * kFPtLd + rl];
-          const int rg = r0 + rl;
-          float4* dst = reinterpret_cast<float4*>(L + (size_t)rg * n + k0 + 8 * c);
-          dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-          dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-          if (k + 1 < N) panel_copy_store<MODE>(W0, W1, N, k, rg, c, v);
+        for (int it = 0; it < kFM * 16 / kFThreads; ++it) {
+          const int item = tid + kFThreads * it, rl = item >> 4, ch = item & 15;
+          if (rl >= first && rl < vr)
+            *reinterpret_cast<float4*>(L + (size_t)(r0 + rl) * n + k0 + 4 * ch) = *x_chunk(PtT, rl, ch);
+        }
+        if (k + 1 < N) {
+#pragma unroll
+          for (int it = 0; it < kFM * 8 / kFThreads; ++it) {
+            const int item = tid + kFThreads * it, rl = item >> 3, c = item & 7;
+            const float4 x0 = *x_chunk(PtT, rl, 2 * c), x1 = *x_chunk(PtT, rl, 2 * c + 1);
+            const float v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+            if (rl >= first && rl < vr) panel_copy_store<MODE>(W0, W1, N, k, r0 + rl, c, v);
+          }
         }
         __syncthreads();
       }

@@ -404,18 +404,20 @@ __device__ void ws_consumers(const WsBars& br, uint8_t* sm, const float* a, floa
           cbar();
         }
         if (diag_only) continue;
-        // (c) X = P T^T (triangle skipped), then L and the tensor-core copy from X^T.
-        xgemm_tri_inplace(PtT, kWPtLd, dg.T, kD64Ld, cbar);
-        // Output: first the tensor-core copy, published to the producer's bulk
-        // copies (the proxy fence then covers only these stores), then L.
-        float v[4][8];
+        // (c) X = P T^T (triangle skipped), then L and the tensor-core copy.
+        xgemm_tri(PtT, kWPtLd, dg.T, kD64Ld, cbar);
+        // Output, lines at a time: first the tensor-core copy, published to the
+        // producer's bulk copies (the proxy fence then covers only these
+        // stores), then L.
+        const int first = mt == 0 ? 64 : 0;  // rows above are the diagonal block's
+        if (k + 1 < N) {
 #pragma unroll
-        for (int it = 0; it < 4; ++it) {
-          const int item = tid + kWConsumers * it;
-          const int rl = item & (kWM - 1), c = item >> 7;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[it][j] = PtT[(8 * c + j) * kWPtLd + rl];
-          if (k + 1 < N && rl < vr && !(mt == 0 && rl < 64)) panel_copy_store<MODE>(W0, W1, N, k, r0 + rl, c, v[it]);
+          for (int it = 0; it < kWM * 8 / kWConsumers; ++it) {
+            const int item = tid + kWConsumers * it, rl = item >> 3, c = item & 7;
+            const float4 x0 = *x_chunk(PtT, rl, 2 * c), x1 = *x_chunk(PtT, rl, 2 * c + 1);
+            const float v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+            if (rl >= first && rl < vr) panel_copy_store<MODE>(W0, W1, N, k, r0 + rl, c, v);
+          }
         }
         umma::fence_proxy_async_all();
         cbar();
@@ -426,13 +428,10 @@ __device__ void ws_consumers(const WsBars& br, uint8_t* sm, const float* a, floa
           for (int q = 0; q < CL; ++q) st_release_cluster(br.tile_done + mt, (uint32_t)q, done);
         }
 #pragma unroll
-        for (int it = 0; it < 4; ++it) {
-          const int item = tid + kWConsumers * it;
-          const int rl = item & (kWM - 1), c = item >> 7;
-          if (rl >= vr || (mt == 0 && rl < 64)) continue;
-          float4* dst = reinterpret_cast<float4*>(L + (size_t)(r0 + rl) * n + k0 + 8 * c);
-          dst[0] = make_float4(v[it][0], v[it][1], v[it][2], v[it][3]);
-          dst[1] = make_float4(v[it][4], v[it][5], v[it][6], v[it][7]);
+        for (int it = 0; it < kWM * 16 / kWConsumers; ++it) {
+          const int item = tid + kWConsumers * it, rl = item >> 4, ch = item & 15;
+          if (rl >= first && rl < vr)
+            *reinterpret_cast<float4*>(L + (size_t)(r0 + rl) * n + k0 + 4 * ch) = *x_chunk(PtT, rl, ch);
         }
         cbar();
       }
