@@ -132,16 +132,18 @@ struct WsBars {
 };
 
 // ---------------------------------------------------------------------------
-// Producer: one thread.
+// Producer: one warp, every decision the same in all lanes, an elected lane
+// issuing.
 template <int MODE, int CL>
 __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t batch, int n, uint32_t tmem,
                             int rank) {
   const int N = n / kWB;
   const size_t rbytes = panel_copy_region_bytes(n);
-  uint32_t n_load[2] = {0u, 0u}, n_empty[2] = {0u, 0u};
+  uint32_t n_load[2] = {0u, 0u};
   int writes[kWMaxSlots] = {0, 0, 0, 0, 0, 0, 0, 0};
   int64_t biter = 0;
   bool ok = true;
+  auto all = [](bool got) { return __all_sync(0xffffffffu, got) != 0; };
   for (int64_t b = blockIdx.x / CL; b < batch && ok; b += gridDim.x / CL, ++biter) {
     const uint8_t* W0 = ws + (size_t)b * 2 * rbytes;
     const uint8_t* W1 = W0 + rbytes;
@@ -162,7 +164,7 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
           // Tile t completes once per block column it exists in (N - 2t per
           // matrix); column k-1 of this matrix is completion number target.
           const int target = (int)(biter * (int64_t)(N - 2 * t) + k);
-          if (!ws_wait_count(br.tile_done + t, target, br.flag, block)) return false;
+          if (!all(ws_wait_count(br.tile_done + t, target, br.flag, block))) return false;
         }
         return true;
       };
@@ -171,7 +173,7 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
         const int s = i & 1;
         if (n_load[s] > 0) {
           // The stage held the previous chunk: wait until the MMAs that read it completed.
-          if (!ws_wait(br.empty + s, (n_load[s] - 1u) & 1u, br.flag)) return false;
+          if (!all(ws_wait(br.empty + s, (n_load[s] - 1u) & 1u, br.flag))) return false;
         }
         if (kc == k - 1 && !deps_ready(mt, true)) return false;
         const int r0 = k0 + mt * kWM;
@@ -179,11 +181,13 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
         const size_t aoff = panel_copy_row_byte(N, kc, r0);
         const size_t boff = panel_copy_row_byte(N, kc, k0);
         uint8_t* st = sm + s * kWStage;
-        umma::mbar_arrive_expect_tx(br.full + s, 2 * abytes + 2 * 8192u);
-        umma::bulk_g2s(st, W0 + aoff, abytes, br.full + s);
-        umma::bulk_g2s(st + 16384, W1 + aoff, abytes, br.full + s);
-        umma::bulk_g2s(st + kWStageA, W0 + boff, 8192u, br.full + s);
-        umma::bulk_g2s(st + kWStageA + 8192, W1 + boff, 8192u, br.full + s);
+        if (umma::elect_one()) {
+          umma::mbar_arrive_expect_tx(br.full + s, 2 * abytes + 2 * 8192u);
+          umma::bulk_g2s(st, W0 + aoff, abytes, br.full + s);
+          umma::bulk_g2s(st + 16384, W1 + aoff, abytes, br.full + s);
+          umma::bulk_g2s(st + kWStageA, W0 + boff, 8192u, br.full + s);
+          umma::bulk_g2s(st + kWStageA + 8192, W1 + boff, 8192u, br.full + s);
+        }
         ++n_load[s];
         return true;
       };
@@ -205,20 +209,19 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
             prefetched = true;
           }
         }
-        if (!ws_wait(br.full + s, (n_load[s] - 1u) & 1u, br.flag)) { ok = false; break; }
+        if (!all(ws_wait(br.full + s, (n_load[s] - 1u) & 1u, br.flag))) { ok = false; break; }
         if (kc == 0 && writes[slot] > 0) {
           // TMEM slot `slot` must have been read by the consumers.
-          if (!ws_wait(br.acc_free + slot, (uint32_t)((writes[slot] - 1) & 1), br.flag)) { ok = false; break; }
+          if (!all(ws_wait(br.acc_free + slot, (uint32_t)((writes[slot] - 1) & 1), br.flag))) { ok = false; break; }
         }
         umma::fence_after_sync();
         const uint32_t st = umma::smem_u32(sm + s * kWStage);
-        panel_copy_mmas<MODE>(tmem + (uint32_t)(kWB * slot), st, st + kWStageA, kc > 0);
-        umma::mma_commit(br.empty + s);
-        ++n_empty[s];
-        if (kc == k - 1) {
-          umma::mma_commit(br.acc_ready + slot);
-          ++writes[slot];
+        if (umma::elect_one()) {
+          panel_copy_mmas<MODE>(tmem + (uint32_t)(kWB * slot), st, st + kWStageA, kc > 0);
+          umma::mma_commit(br.empty + s);
+          if (kc == k - 1) umma::mma_commit(br.acc_ready + slot);
         }
+        if (kc == k - 1) ++writes[slot];
         if (!prefetched && next == i + 1 && next < iters) {
           if (!issue_load(next)) { ok = false; break; }
           ++next;
@@ -231,7 +234,7 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
   for (int s = 0; s < 2; ++s) {
     if (n_load[s] > 0) umma::mbar_wait_bounded(br.full + s, (n_load[s] - 1u) & 1u, kWPolls);
   }
-  umma::mma_commit(br.drain);
+  if (umma::elect_one()) umma::mma_commit(br.drain);
   umma::mbar_wait_bounded(br.drain, 0u, kWPolls);
 }
 
@@ -498,7 +501,7 @@ __global__ void __launch_bounds__(kWThreads, 1)
   const uint32_t tmem = *br.tslot;
   const int rank = CL > 1 ? (int)umma::cluster_rank() : 0;
   if (warp == kWConsumers / 32) {
-    if ((tid & 31) == 0) ws_producer<MODE, CL>(br, sm, ws, batch, n, tmem, rank);
+    ws_producer<MODE, CL>(br, sm, ws, batch, n, tmem, rank);
   } else {
     ws_consumers<MODE, CL>(br, sm, a, l, ws, batch, n, tmem, info, rank, grd);
   }
