@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kGThreads, 2) gemm_tc_kernel(GemmArgs g, int t
       umma::fence_proxy_async_smem();
       umma::fence_before_sync();
       __syncthreads();
-      if (tid == 0) {
+      if (warp == 0 && umma::elect_one()) {
         umma::fence_after_sync();
         g_mmas<MODE>(tmem, umma::smem_u32(opA), umma::smem_u32(opB), any);
         umma::mma_commit(mbar);
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(kBThreads, 1) gemm_bulk_kernel(GemmArgs g, int
 
   if (warp == kBEpi / 32) {
     // ---------------- producer / MMA issuer ----------------
-    if (lane == 0) {
+    if (umma::elect_one()) {
       uint32_t gload = 0, guse = 0;
       bool ok = true;
       // Loader cursor: the next chunk to bring in (item lw, chunk lc).

@@ -59,7 +59,7 @@ constexpr uint32_t kFSmemBytes = kFZeroOff + kFZeroBytes + 1024;
 constexpr uint32_t kFSmemOneCta = 120 * 1024;  // forces one CTA per SM (512 TMEM columns)
 
 constexpr uint32_t kNoTmem = 0xffffffffu;
-constexpr int kFStripThread = 128;  // warp 4, free during the diagonal engine
+constexpr int kFStripWarp = 4;  // free during the diagonal engine
 
 // One thread's 32 values of P = A - D for row r0 + rl (rl < 0: beyond the
 // matrix, zeros) and columns k0 + 32 h .. + 31, D from the TMEM columns at
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(kFThreads, 2)
       const int mtiles = (n - k0 + kFM - 1) / kFM;
       // ---------------- phase 1: left-looking update into TMEM -------------
       if (k > 0) {
-        if (tid == 0) {
+        if (warp == 0 && umma::elect_one()) {
           const int iters = mtiles * k;
           auto load = [&](int i, int s) {
             const int mt = i / k, kc = i - (i / k) * k;
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kFThreads, 2)
             // Zero strip right of the diagonal block: one bulk store per row
             // from the zero buffer, issued by one thread and left to run.
             const uint32_t strip = 4u * (uint32_t)(n - k0 - kFB);
-            if (tid == kFStripThread && strip > 0) {
+            if (strip > 0 && warp == kFStripWarp && umma::elect_one()) {
               for (int r = 0; r < 64; ++r)
                 umma::bulk_s2g(L + (size_t)(k0 + r) * n + k0 + kFB, sm + kFZeroOff, strip);
               umma::bulk_commit();
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kFThreads, 2)
   if (grd.state != nullptr && tid == 0)
     for (; b < batch; b += gridDim.x) grd.state[b] = -1;
   // The strip's bulk stores read the zero buffer until they complete.
-  if (tid == kFStripThread) umma::bulk_wait_all();
+  if (warp == kFStripWarp && umma::elect_one()) umma::bulk_wait_all();
   // Release TMEM after a last bounded chance for outstanding MMAs.
   if (!ok) {
     umma::mbar_wait_bounded(done, ph_done, kFPolls);

@@ -69,7 +69,7 @@ constexpr int kWMaxSlots = 8;                   // TMEM accumulator slots (512 c
 constexpr uint32_t kWSmemBytes = kWCntOff + 4 * kWMaxTiles + 1024;
 
 using ConsumerBar = NamedBarrier1<kWConsumers>;
-constexpr int kWStripThread = 128;  // consumer warp 4, free during the diagonal engine
+constexpr int kWStripWarp = 4;  // a consumer warp, free during the diagonal engine
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smem_u32(mbar)) : "memory");
@@ -339,7 +339,7 @@ __device__ void ws_consumers(const WsBars& br, uint8_t* sm, const float* a, floa
             // Zero strip right of the diagonal block: one bulk store per row
             // from the zero buffer, issued by one thread and left to run.
             const uint32_t strip = 4u * (uint32_t)(n - k0 - kWB);
-            if (tid == kWStripThread && rank == 0 && strip > 0) {
+            if (rank == 0 && strip > 0 && warp == kWStripWarp && umma::elect_one()) {
               for (int r = 0; r < 64; ++r) {
                 uint8_t* row = reinterpret_cast<uint8_t*>(L + (size_t)(k0 + r) * n + k0 + kWB);
                 for (uint32_t off = 0; off < strip; off += kWZeroBytes)
@@ -453,7 +453,7 @@ __device__ void ws_consumers(const WsBars& br, uint8_t* sm, const float* a, floa
     }
   }
   // The strip's bulk stores read the zero buffer until they complete.
-  if (tid == kWStripThread) umma::bulk_wait_all();
+  if (warp == kWStripWarp && umma::elect_one()) umma::bulk_wait_all();
 }
 
 template <int MODE, int CL>

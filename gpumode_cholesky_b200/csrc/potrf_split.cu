@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kUThreads, 2)
   umma::fence_after_sync();
   const uint32_t tmem = *tslot;
 
-  if (tid == 0) {
+  if (warp == 0 && umma::elect_one()) {
     bool ok = true;
     uint32_t ph_full[2] = {0u, 0u};
     uint32_t n_empty[2] = {0u, 0u};
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(kXThreads, 1)
 
   if (warp == kXConsumers / 32) {
     // ---------------- producer / MMA issuer ----------------
-    if (lane == 0) {
+    if (umma::elect_one()) {
       int64_t gi = 0, loaded = 0;  // panels consumed / loaded (all items)
       int64_t gc = 0;              // chunks started
       bool ok = true;
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(kXThreads, 1)
 
 // ---- step kernel -------------------------------------------------------------
 constexpr int kSThreads = 128;
-constexpr int kSStripThread = 96;  // warp 3 lane 0
+constexpr int kSStripWarp = 3;
 // Panel k-1 rows k0..k0+63: the B operand (region 0 at +0, region 1 at
 // +8 KB), and also the diagonal product's A operand (A1 = 8 KB: its rows
 // 64..127, whose accumulator lanes nobody reads, overlap what follows).
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(kSThreads, 2)
       const bool own = q < chunks;
       const int r0 = k0 + 64 + q * kSThreads;
       const uint32_t vr = own ? (uint32_t)min(kSThreads, n - r0) : 0u;
-      if (tid == 0) {
+      if (warp == 0 && umma::elect_one()) {
         const size_t boff = panel_copy_row_byte(N, k - 1, k0);
         umma::mbar_arrive_expect_tx(full, (first ? 2u * 8192u : 0u) + 2u * vr * 128u);
         if (first) {
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(kSThreads, 2)
     // 2. Zero strip right of the diagonal block: rows g, g + G, ... of it as
     //    bulk stores from the zero buffer, issued by warp 3 (idle in the
     //    P_kk formation and the diagonal factor) and left to run.
-    if (tid == kSStripThread) {
+    if (warp == kSStripWarp && umma::elect_one()) {
       const uint32_t strip = 4u * (uint32_t)(n - k0 - 64);
       if (strip > 0) {
         for (int r = g; r < 64; r += G) {
@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(kSThreads, 2)
       if (job % G == 0) grd.state[job / G] = -1;
   if (!ok) umma::mbar_wait_bounded(done, ph_done, kSplitPolls);
   // The strip's bulk stores read the zero buffer until they complete.
-  if (tid == kSStripThread) umma::bulk_wait_all();
+  if (warp == kSStripWarp && umma::elect_one()) umma::bulk_wait_all();
   umma::fence_before_sync();
   __syncthreads();
   if (upd && warp == 0) umma::tmem_dealloc(tmem, kSTmemCols);

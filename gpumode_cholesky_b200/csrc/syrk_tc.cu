@@ -152,7 +152,7 @@ __device__ __forceinline__ bool tc_run(const TcShared& sh, uint32_t tmem, bool s
   umma::fence_proxy_async_smem();
   umma::fence_before_sync();
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32 && umma::elect_one()) {
     umma::fence_after_sync();
     issue_mmas<MODE>(tmem, sh.opA, same_operand ? sh.opA : sh.opB);
     umma::mma_commit(sh.mbar);
