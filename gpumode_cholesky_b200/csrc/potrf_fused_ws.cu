@@ -133,7 +133,10 @@ struct WsBars {
 
 // ---------------------------------------------------------------------------
 // Producer: one warp, every decision the same in all lanes, an elected lane
-// issuing.
+// issuing.  Chunks (a tile's product over one earlier block column) are counted
+// along, not divided out of an index: with one warp and two stages, all that is
+// between two chunks' MMAs adds to the update (60 x 1024: 494 -> 479 us; the
+// packed list of 400 orders up to 2048: 4246 -> 3942).
 template <int MODE, int CL>
 __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t batch, int n, uint32_t tmem,
                             int rank) {
@@ -168,9 +171,11 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
         }
         return true;
       };
-      auto issue_load = [&](int i) -> bool {
-        const int mt = ws_tile_of<CL>(i / k, rank), kc = i - (i / k) * k;
-        const int s = i & 1;
+      // The next chunk to load: entry lj of the tile list, column lkc.
+      int next = 0, lj = 0, lkc = 0;
+      auto issue_load = [&]() -> bool {
+        const int mt = ws_tile_of<CL>(lj, rank), kc = lkc;
+        const int s = next & 1;
         if (n_load[s] > 0) {
           // The stage held the previous chunk: wait until the MMAs that read it completed.
           if (!all(ws_wait(br.empty + s, (n_load[s] - 1u) & 1u, br.flag))) return false;
@@ -189,25 +194,24 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
           umma::bulk_g2s(st + kWStageA + 8192, W1 + boff, 8192u, br.full + s);
         }
         ++n_load[s];
+        ++next;
+        if (++lkc == k) {
+          lkc = 0;
+          ++lj;
+        }
         return true;
       };
-      int next = 0;
-      if (iters > 0) {
-        if (!issue_load(0)) { ok = false; break; }
-        next = 1;
+      if (iters > 0 && !issue_load()) {
+        ok = false;
+        break;
       }
+      int slot = 0, kc = 0;
       for (int i = 0; i < iters && ok; ++i) {
         const int s = i & 1;
-        const int slot = i / k, kc = i - (i / k) * k;
         // Prefetch the next chunk unless it would wait on consumers.
-        bool prefetched = false;
-        if (next == i + 1 && next < iters) {
-          const int nmt = ws_tile_of<CL>(next / k, rank), nkc = next - (next / k) * k;
-          if (nkc != k - 1 || deps_ready(nmt, false)) {
-            if (!issue_load(next)) { ok = false; break; }
-            ++next;
-            prefetched = true;
-          }
+        if (next < iters && (lkc != k - 1 || deps_ready(ws_tile_of<CL>(lj, rank), false)) && !issue_load()) {
+          ok = false;
+          break;
         }
         if (!all(ws_wait(br.full + s, (n_load[s] - 1u) & 1u, br.flag))) { ok = false; break; }
         if (kc == 0 && writes[slot] > 0) {
@@ -222,9 +226,13 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
           if (kc == k - 1) umma::mma_commit(br.acc_ready + slot);
         }
         if (kc == k - 1) ++writes[slot];
-        if (!prefetched && next == i + 1 && next < iters) {
-          if (!issue_load(next)) { ok = false; break; }
-          ++next;
+        if (++kc == k) {
+          kc = 0;
+          ++slot;
+        }
+        if (next == i + 1 && next < iters && !issue_load()) {
+          ok = false;
+          break;
         }
       }
     }
