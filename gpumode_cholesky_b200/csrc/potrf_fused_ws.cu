@@ -142,8 +142,9 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
                             int rank) {
   const int N = n / kWB;
   const size_t rbytes = panel_copy_region_bytes(n);
-  uint32_t n_load[2] = {0u, 0u};
-  int writes[kWMaxSlots] = {0, 0, 0, 0, 0, 0, 0, 0};
+  // Bit s: stage s has been loaded; parity of its number of loads.  Likewise
+  // the writes into each TMEM slot.
+  uint32_t loaded = 0u, load_par = 0u, written = 0u, write_par = 0u;
   int64_t biter = 0;
   bool ok = true;
   auto all = [](bool got) { return __all_sync(0xffffffffu, got) != 0; };
@@ -176,9 +177,9 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
       auto issue_load = [&]() -> bool {
         const int mt = ws_tile_of<CL>(lj, rank), kc = lkc;
         const int s = next & 1;
-        if (n_load[s] > 0) {
+        if ((loaded >> s) & 1u) {
           // The stage held the previous chunk: wait until the MMAs that read it completed.
-          if (!all(ws_wait(br.empty + s, (n_load[s] - 1u) & 1u, br.flag))) return false;
+          if (!all(ws_wait(br.empty + s, ((load_par >> s) & 1u) ^ 1u, br.flag))) return false;
         }
         if (kc == k - 1 && !deps_ready(mt, true)) return false;
         const int r0 = k0 + mt * kWM;
@@ -193,7 +194,8 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
           umma::bulk_g2s(st + kWStageA, W0 + boff, 8192u, br.full + s);
           umma::bulk_g2s(st + kWStageA + 8192, W1 + boff, 8192u, br.full + s);
         }
-        ++n_load[s];
+        loaded |= 1u << s;
+        load_par ^= 1u << s;
         ++next;
         if (++lkc == k) {
           lkc = 0;
@@ -213,10 +215,10 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
           ok = false;
           break;
         }
-        if (!all(ws_wait(br.full + s, (n_load[s] - 1u) & 1u, br.flag))) { ok = false; break; }
-        if (kc == 0 && writes[slot] > 0) {
+        if (!all(ws_wait(br.full + s, ((load_par >> s) & 1u) ^ 1u, br.flag))) { ok = false; break; }
+        if (kc == 0 && ((written >> slot) & 1u)) {
           // TMEM slot `slot` must have been read by the consumers.
-          if (!all(ws_wait(br.acc_free + slot, (uint32_t)((writes[slot] - 1) & 1), br.flag))) { ok = false; break; }
+          if (!all(ws_wait(br.acc_free + slot, ((write_par >> slot) & 1u) ^ 1u, br.flag))) { ok = false; break; }
         }
         umma::fence_after_sync();
         const uint32_t st = umma::smem_u32(sm + s * kWStage);
@@ -225,7 +227,10 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
           umma::mma_commit(br.empty + s);
           if (kc == k - 1) umma::mma_commit(br.acc_ready + slot);
         }
-        if (kc == k - 1) ++writes[slot];
+        if (kc == k - 1) {
+          written |= 1u << slot;
+          write_par ^= 1u << slot;
+        }
         if (++kc == k) {
           kc = 0;
           ++slot;
@@ -240,7 +245,7 @@ __device__ void ws_producer(const WsBars& br, uint8_t* sm, uint8_t* ws, int64_t 
   if (!ok) *br.flag = 1;
   // Drain: every copy lands and every MMA completes before TMEM is released.
   for (int s = 0; s < 2; ++s) {
-    if (n_load[s] > 0) umma::mbar_wait_bounded(br.full + s, (n_load[s] - 1u) & 1u, kWPolls);
+    if ((loaded >> s) & 1u) umma::mbar_wait_bounded(br.full + s, ((load_par >> s) & 1u) ^ 1u, kWPolls);
   }
   if (umma::elect_one()) umma::mma_commit(br.drain);
   umma::mbar_wait_bounded(br.drain, 0u, kWPolls);
