@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(kFThreads, 2)
   const uint32_t tmem = *tslot;
 
   // mbarrier phase bookkeeping (thread 0 drives full/empty; all wait on done)
-  uint32_t ph_full[2] = {0u, 0u};
-  uint32_t n_empty[2] = {0u, 0u};
+  // Bit s: parity of stage s's next phase.
+  uint32_t ph_full = 0u, ph_empty = 0u;
   uint32_t ph_done = 0u;
   bool ok = true;
 
@@ -151,47 +151,55 @@ __global__ void __launch_bounds__(kFThreads, 2)
       if (k > 0) {
         if (warp == 0 && umma::elect_one()) {
           const int iters = mtiles * k;
-          auto load = [&](int i, int s) {
-            const int mt = i / k, kc = i - (i / k) * k;
-            const int r0 = k0 + mt * kFM;
+          // The next chunk to load (row tile, earlier column), and the one in use.
+          int lt = 0, lkc = 0, mt = 0, kc = 0;
+          auto load = [&](int s) {
+            const int r0 = k0 + lt * kFM;
             const uint32_t abytes = (uint32_t)min(kFM, n - r0) * 128u;
-            const size_t aoff = panel_copy_row_byte(N, kc, r0);
-            const size_t boff = panel_copy_row_byte(N, kc, k0);
+            const size_t aoff = panel_copy_row_byte(N, lkc, r0);
+            const size_t boff = panel_copy_row_byte(N, lkc, k0);
             uint8_t* st = sm + s * kFStage;
             umma::mbar_arrive_expect_tx(full + s, 2 * abytes + 2 * 8192u);
             umma::bulk_g2s(st, W0 + aoff, abytes, full + s);
             umma::bulk_g2s(st + 16384, W1 + aoff, abytes, full + s);
             umma::bulk_g2s(st + kFStageA, W0 + boff, 8192u, full + s);
             umma::bulk_g2s(st + kFStageA + 8192, W1 + boff, 8192u, full + s);
+            if (++lkc == k) {
+              lkc = 0;
+              ++lt;
+            }
           };
           int loaded = 0;
-          load(0, 0);
+          load(0);
           ++loaded;
           if (iters > 1) {
-            load(1, 1);
+            load(1);
             ++loaded;
           }
           int waited = 0;
           for (int i = 0; i < iters; ++i) {
             const int s = i & 1;
-            if (!umma::mbar_wait_bounded(full + s, ph_full[s], kFPolls)) {
+            if (!umma::mbar_wait_bounded(full + s, (ph_full >> s) & 1u, kFPolls)) {
               ok = false;
               break;
             }
-            ph_full[s] ^= 1u;
+            ph_full ^= 1u << s;
             ++waited;
             umma::fence_after_sync();
-            const int mt = i / k, kc = i - (i / k) * k;
             const uint32_t st = umma::smem_u32(sm + s * kFStage);
             panel_copy_mmas<MODE>(tmem + (uint32_t)(kFB * mt), st, st + kFStageA, kc > 0);
             umma::mma_commit(empty + s);
-            ++n_empty[s];
+            if (++kc == k) {
+              kc = 0;
+              ++mt;
+            }
             if (i + 2 < iters) {
-              if (!umma::mbar_wait_bounded(empty + s, (n_empty[s] - 1u) & 1u, kFPolls)) {
+              if (!umma::mbar_wait_bounded(empty + s, (ph_empty >> s) & 1u, kFPolls)) {
                 ok = false;
                 break;
               }
-              load(i + 2, s);
+              ph_empty ^= 1u << s;
+              load(s);
               ++loaded;
             }
           }
@@ -201,7 +209,8 @@ __global__ void __launch_bounds__(kFThreads, 2)
             for (int s = 0; s < 2; ++s) {
               const int last = iters - 1 - ((iters - 1 - s) & 1);  // last iteration using stage s
               if (last >= 0 && last + 2 >= iters) {
-                if (!umma::mbar_wait_bounded(empty + s, (n_empty[s] - 1u) & 1u, kFPolls)) ok = false;
+                if (!umma::mbar_wait_bounded(empty + s, (ph_empty >> s) & 1u, kFPolls)) ok = false;
+                ph_empty ^= 1u << s;
               }
             }
           }
@@ -209,7 +218,7 @@ __global__ void __launch_bounds__(kFThreads, 2)
             // Let the copies still in flight land before anything else runs.
             for (int i = waited; i < loaded; ++i) {
               const int s = i & 1;
-              if (umma::mbar_wait_bounded(full + s, ph_full[s], kFPolls)) ph_full[s] ^= 1u;
+              if (umma::mbar_wait_bounded(full + s, (ph_full >> s) & 1u, kFPolls)) ph_full ^= 1u << s;
             }
             *flag = 1;
           }

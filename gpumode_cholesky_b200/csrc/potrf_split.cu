@@ -115,8 +115,7 @@ __global__ void __launch_bounds__(kUThreads, 2)
 
   if (warp == 0 && umma::elect_one()) {
     bool ok = true;
-    uint32_t ph_full[2] = {0u, 0u};
-    uint32_t n_empty[2] = {0u, 0u};
+    uint32_t ph_full = 0u, ph_empty = 0u;  // bit st: parity of the stage's next phase
     auto load = [&](int i, int st) {
       const int c = c_lo + i;
       const uint32_t abytes = (uint32_t)vr * 128u;
@@ -138,23 +137,23 @@ __global__ void __launch_bounds__(kUThreads, 2)
     }
     for (int i = 0; i < iters; ++i) {
       const int st = i & 1;
-      if (!umma::mbar_wait_bounded(full + st, ph_full[st], kSplitPolls)) {
+      if (!umma::mbar_wait_bounded(full + st, (ph_full >> st) & 1u, kSplitPolls)) {
         ok = false;
         break;
       }
-      ph_full[st] ^= 1u;
+      ph_full ^= 1u << st;
       ++waited;
       umma::fence_after_sync();
       const uint32_t sa = umma::smem_u32(sm + st * kUStage);
       panel_copy_mmas<MODE>(tmem, sa, sa + kUStageA, i > 0);
       umma::mma_commit(empty + st);
-      ++n_empty[st];
       if (i + 2 < iters) {
         // Stage st is reused only once the MMAs reading it have completed.
-        if (!umma::mbar_wait_bounded(empty + st, (n_empty[st] - 1u) & 1u, kSplitPolls)) {
+        if (!umma::mbar_wait_bounded(empty + st, (ph_empty >> st) & 1u, kSplitPolls)) {
           ok = false;
           break;
         }
+        ph_empty ^= 1u << st;
         load(i + 2, st);
         ++loaded;
       }
@@ -163,7 +162,7 @@ __global__ void __launch_bounds__(kUThreads, 2)
       // Let copies still in flight land before the staging area is reused.
       for (int i = waited; i < loaded; ++i) {
         const int st = i & 1;
-        if (umma::mbar_wait_bounded(full + st, ph_full[st], kSplitPolls)) ph_full[st] ^= 1u;
+        if (umma::mbar_wait_bounded(full + st, (ph_full >> st) & 1u, kSplitPolls)) ph_full ^= 1u << st;
       }
       *flag = 1;
     }
