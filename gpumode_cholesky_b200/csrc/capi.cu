@@ -5,9 +5,9 @@
 //   n <= 32    one warp per matrix            (potrf_warp32_kernel)
 //   n <= 128   one CTA per matrix, in smem    (potrf_cta128_kernel)
 //   n >  128   tensor modes, n % 64 == 0 (choose_path):
-//                many CTAs per matrix when n > 1024 or the batch is too
-//                small to fill the GPU one CTA per matrix (potrf_split);
-//                else one CTA per matrix (potrf_fused / potrf_fused_ws);
+//                many CTAs per matrix when n > 1024 (potrf_split); else one
+//                CTA per matrix, or a cluster when the batch is too small to
+//                fill the GPU (potrf_fused / potrf_fused_ws);
 //              FP32: tile tasks in one launch (potrf_tiles); any other n or
 //              FP64 diagonal tiles: blocked right-looking (potrf_blocked)
 // There is no CPU path and no vendor-library fallback.
@@ -83,14 +83,18 @@ bool path_supported(int path, int64_t batch, int64_t n, int mode) {
 }
 
 // The n > 128 algorithm for (batch, n, mode).  Tensor modes, measured on
-// B200 (BF16x3): up to n = 1024 one CTA per matrix while the batch fills
-// the GPU (640x512: 1225 us), else the warp-specialized kernel in clusters of
-// up to 8 CTAs per matrix (60x1024: 646 us, 4x1024: 421 us); above 1024 the
-// multi-CTA split path (8x2048: 1351 us).  FP32: blocked (which is
-// potrf_tiles but for FP64 diagonal tiles).
+// B200 (BF16x3, us, one CTA per matrix / warp-specialized / split).  Up to n =
+// 512, where two CTAs share an SM, one CTA per matrix while the batch fills the
+// GPU (640x512: 838 / 1018 / 1252; 200x512: 320 / 412 / 508), else the
+// warp-specialized kernel in clusters of up to 8 CTAs per matrix (148x512: 220 /
+// 214 / 491; 16x512: 205 / 134 / 158).  Up to 1024 one CTA has the SM (TMEM) in
+// both, so the warp-specialized kernel at every batch (148x1024: 900 / 759 /
+// 1844; 200x768: 908 / 839 / 1149; 60x1024: 785 / 467 / 675; 4x1024: 738 / 312 /
+// 321).  Above 1024 the multi-CTA split path (8x2048: 727).  FP32: blocked (which
+// is potrf_tiles but for FP64 diagonal tiles).
 int choose_path(int64_t batch, int64_t n, int mode) {
   const int64_t sms = device_sms();
-  if (fused_supported(n, mode)) return batch > sms ? B2P_PATH_FUSED : B2P_PATH_FUSED_WS;
+  if (fused_supported(n, mode)) return batch > sms && n <= 512 ? B2P_PATH_FUSED : B2P_PATH_FUSED_WS;
   if (split_supported(n, mode)) return B2P_PATH_SPLIT;
   return B2P_PATH_BLOCKED;
 }
@@ -214,15 +218,16 @@ int b2p_potrf_batched_ex(const float* a, float* l, int64_t batch, int64_t n, int
     return set_error(B2P_ERR_UNSUPPORTED, "path %d does not support n=%lld mode 0x%x", path, (long long)n, mode);
   int st = B2P_OK;
   bool done = false;
-  if (auto_path && path == B2P_PATH_FUSED) {
+  if (auto_path && (path == B2P_PATH_FUSED || path == B2P_PATH_FUSED_WS)) {
     // One CTA per matrix runs in waves of `per` matrices; when the last wave
     // would be less than half full, those matrices run instead as clusters
-    // of CTAs each (same workspace layout, so they take their own slice).
+    // of CTAs each (same workspace layout, so they take their own slice;
+    // 640x512 838 -> 798 us, 160x1024 1452 -> 1076).
     const int64_t per = (int64_t)device_sms() * (n <= 512 ? 2 : 1);
     const int64_t tail = batch % per;
     if (batch > per && tail > 0 && tail * 2 <= per && fused_ws_supported(tail, n, mode)) {
       const int64_t head = batch - tail;
-      st = potrf_fused(a, l, head, (int)n, mode, workspace, workspace_bytes, info, s, grd);
+      st = potrf_path(a, l, head, (int)n, mode, path, workspace, workspace_bytes, info, s, grd);
       if (st == B2P_OK) {
         const size_t moff = (size_t)head * (size_t)n * (size_t)n;
         const size_t woff = (size_t)head * 2 * panel_copy_region_bytes((int)n);

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kFThreads, 2)
         umma::fence_before_sync();
         __syncthreads();
         if (mt == 0) {
-          // L_kk and T^T (T = L_kk^{-1}, in dg.T) from the pipelined engine
+          // L_kk and T^T (T = L_kk^{-1}, in dg.T) from the diagonal engine
           // on warps 0-3.  Meanwhile warps 4-7 form P = A - D of the later
           // row tiles (their loads of A hide behind the diagonal engine) and
           // park it in place of D in TMEM, each warp its lane quarter.

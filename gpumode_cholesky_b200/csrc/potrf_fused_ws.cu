@@ -5,9 +5,9 @@
 // update of block column k+1 runs concurrently with the panel work of block
 // column k:
 //
-//   warp 8 (producer, one thread)  streams the panel copies with
-//        cp.async.bulk (two stages) and issues the tcgen05 MMAs of the next
-//        block column tile by tile; per tile it commits `acc_ready`;
+//   warp 8 (producer)  streams the panel copies with cp.async.bulk (two
+//        stages) and issues the tcgen05 MMAs of the next block column tile by
+//        tile; per tile it commits `acc_ready`;
 //   warps 0-7 (consumers)  per tile: wait `acc_ready`, read D from TMEM
 //        (then arrive `acc_free`), P = A - D, factor + invert the diagonal
 //        block (tile 0), X = P T^T in FP32, write L and the tensor-core copy
@@ -340,7 +340,7 @@ __device__ void ws_consumers(const WsBars& br, uint8_t* sm, const float* a, floa
           }
         }
         cbar();
-        // (b) diagonal block: L_kk and T^T (pipelined engine), zero strip.
+        // (b) diagonal block: L_kk and T^T (diag64.cuh), zero strip.
         if (mt == 0) {
           // Warps 0-3 run the diagonal engine.  Warps 4-7 meanwhile form
           // P = A - D of this CTA's later tiles of the column (each warp its
@@ -543,7 +543,7 @@ static int ws_cluster_size(int64_t batch, int n) {
 // Orders up to 1024.  Larger ones would fit (clusters big enough for TMEM),
 // but with K up to n every CTA then streams its whole row range of panel
 // copies per block column and is bound by its own bulk-copy bandwidth
-// (8x2048: 1630 us against 1351 us on the split path; 1x4096: 7490 vs 2335).
+// (8x2048: 1090 us against 727 on the split path; 1x4096: 5250 vs 1304).
 bool fused_ws_fits(int64_t batch, int64_t n, int mode) {
   const int m = mode & B2P_MODE_MASK;
   return (m == B2P_MODE_TF32 || m == B2P_MODE_BF16X3) && !(mode & B2P_FLAG_FP64_DIAG) && n > 128 && n % 64 == 0 &&
