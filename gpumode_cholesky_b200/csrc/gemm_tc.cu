@@ -37,32 +37,41 @@ __device__ __forceinline__ float g_round_tf32(float x) {
   return __uint_as_float(r);
 }
 
+// Row r, columns 8 c .. 8 c + 7 of an operand image.
+template <int MODE>
+__device__ __forceinline__ void g_put8(uint8_t* op, int r, int c, const float (&v)[8]) {
+  if (MODE == B2P_MODE_TF32) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int Q = 2 * c + q;  // float4 index within the 64-wide row
+      *reinterpret_cast<float4*>(op + (Q >> 3) * 16384 + umma::sw128_offset(r, Q & 7)) =
+          make_float4(g_round_tf32(v[4 * q]), g_round_tf32(v[4 * q + 1]), g_round_tf32(v[4 * q + 2]),
+                      g_round_tf32(v[4 * q + 3]));
+    }
+  } else {
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      __nv_bfloat16 h0, l0, h1, l1;
+      umma::split_bf16(v[2 * q], h0, l0);
+      umma::split_bf16(v[2 * q + 1], h1, l1);
+      hi[q] = umma::pack_bf16(h0, h1);
+      lo[q] = umma::pack_bf16(l0, l1);
+    }
+    const uint32_t off = umma::sw128_offset(r, c);
+    *reinterpret_cast<uint4*>(op + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(op + 16384 + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+}
+
 // Write 64 K values of operand row r into the swizzled tile.
 template <int MODE>
 __device__ __forceinline__ void g_store_row(uint8_t* op, int r, const float (&v)[64]) {
-  if (MODE == B2P_MODE_TF32) {
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const float4 t = make_float4(g_round_tf32(v[4 * q]), g_round_tf32(v[4 * q + 1]), g_round_tf32(v[4 * q + 2]),
-                                   g_round_tf32(v[4 * q + 3]));
-      *reinterpret_cast<float4*>(op + (q >> 3) * 16384 + umma::sw128_offset(r, q & 7)) = t;
-    }
-  } else {
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      uint32_t hi[4], lo[4];
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        __nv_bfloat16 h0, l0, h1, l1;
-        umma::split_bf16(v[8 * c + 2 * p], h0, l0);
-        umma::split_bf16(v[8 * c + 2 * p + 1], h1, l1);
-        hi[p] = umma::pack_bf16(h0, h1);
-        lo[p] = umma::pack_bf16(l0, l1);
-      }
-      const uint32_t off = umma::sw128_offset(r, c);
-      *reinterpret_cast<uint4*>(op + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-      *reinterpret_cast<uint4*>(op + 16384 + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    }
+  for (int c = 0; c < 8; ++c) {
+    const float w[8] = {v[8 * c],     v[8 * c + 1], v[8 * c + 2], v[8 * c + 3],
+                        v[8 * c + 4], v[8 * c + 5], v[8 * c + 6], v[8 * c + 7]};
+    g_put8<MODE>(op, r, c, w);
   }
 }
 
@@ -77,36 +86,52 @@ __device__ __forceinline__ int2 kept_range(int keep, int i, int rows, int k0, in
   const int hi = i >= rows ? 0 : min(min(len, kdim - k0), keep == kKeepUpTo ? i - k0 + 1 : len);
   return make_int2(lo, hi);
 }
+// src[in.x .. in.y - 1] of 8 values, zeros elsewhere.
+__device__ __forceinline__ void g_load8(const float* src, int2 in, float (&v)[8]) {
+  if (in.x == 0 && in.y == 8 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const float4 t = reinterpret_cast<const float4*>(src)[q];
+      v[4 * q] = t.x;
+      v[4 * q + 1] = t.y;
+      v[4 * q + 2] = t.z;
+      v[4 * q + 3] = t.w;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = (q >= in.x && q < in.y) ? src[q] : 0.0f;
+  }
+}
+
 // Operand row `r` (0..127) of a tile: logical element (row0 + r, k0 + kk).
 // `rowmajor`: element (i, kk) at mat[i*ld + kk] (K contiguous) else at
 // mat[kk*ld + i] (rows contiguous across threads: coalesced).
 template <int MODE>
 __device__ __forceinline__ void g_stage(const float* mat, int ld, bool rowmajor, int keep, int rows, int kdim,
                                         int row0, int k0, uint8_t* op, int r) {
-  float v[64];
-  const int i = row0 + r;
-  const int2 in = kept_range(keep, i, rows, k0, kdim, kGK);
   if (rowmajor) {
-    const float* p = mat + (size_t)i * ld + k0;
-    if (in.x == 0 && in.y == kGK && (ld & 3) == 0) {
+    // Eight lanes to a row (thread r of the operand's 128), whole lines read
+    // (a thread per row: 8x512 GP 429 us against 421, 64x256 adjoint 244, 239).
 #pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const float4 t = reinterpret_cast<const float4*>(p)[q];
-        v[4 * q] = t.x;
-        v[4 * q + 1] = t.y;
-        v[4 * q + 2] = t.z;
-        v[4 * q + 3] = t.w;
+    for (int h = 0; h < 2; ++h) {
+      float v[4][8];
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int rl = 16 * (4 * h + it) + (r >> 3), kk = k0 + 8 * (r & 7), i = row0 + rl;
+        g_load8(mat + (size_t)i * ld + kk, kept_range(keep, i, rows, kk, kdim, 8), v[it]);
       }
-    } else {
 #pragma unroll
-      for (int q = 0; q < 64; ++q) v[q] = (q >= in.x && q < in.y) ? p[q] : 0.0f;
+      for (int it = 0; it < 4; ++it) g_put8<MODE>(op, 16 * (4 * h + it) + (r >> 3), r & 7, v[it]);
     }
   } else {
+    float v[64];
+    const int i = row0 + r;
+    const int2 in = kept_range(keep, i, rows, k0, kdim, kGK);
     const float* p = mat + (size_t)k0 * ld + i;
 #pragma unroll
     for (int q = 0; q < 64; ++q) v[q] = (q >= in.x && q < in.y) ? p[(size_t)q * ld] : 0.0f;
+    g_store_row<MODE>(op, r, v);
   }
-  g_store_row<MODE>(op, r, v);
 }
 
 // Row i, columns j0 .. j0 + 31 of the output.
@@ -297,31 +322,6 @@ __global__ void __launch_bounds__(kPThreads) gemm_pack_kernel(const float* __res
   __shared__ __align__(1024) uint8_t image[kGOperand];
   const int tid = threadIdx.x;
   const size_t per = (size_t)((rows + kGT - 1) / kGT) * tiles_k * kGOperand;
-  // Columns 8 c .. 8 c + 7 of row r of the block.
-  auto put = [&](int r, int c, const float (&v)[8]) {
-    if (MODE == B2P_MODE_TF32) {
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int Q = 2 * c + q;  // float4 index within the 64-wide row
-        *reinterpret_cast<float4*>(image + (Q >> 3) * 16384 + umma::sw128_offset(r, Q & 7)) =
-            make_float4(g_round_tf32(v[4 * q]), g_round_tf32(v[4 * q + 1]), g_round_tf32(v[4 * q + 2]),
-                        g_round_tf32(v[4 * q + 3]));
-      }
-    } else {
-      uint32_t hi[4], lo[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        __nv_bfloat16 h0, l0, h1, l1;
-        umma::split_bf16(v[2 * q], h0, l0);
-        umma::split_bf16(v[2 * q + 1], h1, l1);
-        hi[q] = umma::pack_bf16(h0, h1);
-        lo[q] = umma::pack_bf16(l0, l1);
-      }
-      const uint32_t off = umma::sw128_offset(r, c);
-      *reinterpret_cast<uint4*>(image + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-      *reinterpret_cast<uint4*>(image + 16384 + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    }
-  };
   for (int64_t b = blockIdx.y; b < items; b += gridDim.y) {
     const int64_t b1 = b / nb2, b2 = b - (b / nb2) * nb2;
     const float* M = mat + b1 * s1 + b2 * s2;
@@ -334,25 +334,12 @@ __global__ void __launch_bounds__(kPThreads) gemm_pack_kernel(const float* __res
       const int2 in = kept_range(keep, i, rows, k0, kdim, 8);
       float v[8];
       if (rowmajor) {
-        const float* src = M + (size_t)i * ld + k0;
-        if (in.x == 0 && in.y == 8 && ((reinterpret_cast<uintptr_t>(src) & 15u) == 0)) {
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const float4 t = __ldg(reinterpret_cast<const float4*>(src) + q);
-            v[4 * q] = t.x;
-            v[4 * q + 1] = t.y;
-            v[4 * q + 2] = t.z;
-            v[4 * q + 3] = t.w;
-          }
-        } else {
-#pragma unroll
-          for (int q = 0; q < 8; ++q) v[q] = (q >= in.x && q < in.y) ? __ldg(src + q) : 0.0f;
-        }
+        g_load8(M + (size_t)i * ld + k0, in, v);
       } else {
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = (q >= in.x && q < in.y) ? __ldg(M + (size_t)(k0 + q) * ld + i) : 0.0f;
       }
-      put(r, c, v);
+      g_put8<MODE>(image, r, c, v);
     }
     umma::fence_proxy_async_smem();
     __syncthreads();
