@@ -15,7 +15,10 @@
 // reads through per-row progress counters.  Every tile it can wait for has an
 // earlier ticket, so it is finished or being worked on by a running CTA: no
 // task waits for one that has not started, whatever the number of CTAs the
-// GPU runs at a time.  All waits are bounded.
+// GPU runs at a time.  All waits are bounded.  A CTA whose wait gives up takes
+// the tickets away, so that the others leave, and the output is marked: info -1
+// for the whole batch, and NaN on the diagonal of every L, since callers
+// without info have nothing else to see it by.
 //
 // The order of the tickets is also the look-ahead: while column j's diagonal
 // tile is being factored, the CTAs that drew the next columns' tasks
@@ -58,6 +61,7 @@ constexpr int kTlStage = kTlRowHalf + kTlColHalf;
 constexpr size_t kTlSmem = ((sizeof(Diag64Smem) + 127) & ~(size_t)127) + 64;
 constexpr int kTlCtasPerSm = 3;
 constexpr uint32_t kTlPolls = 1u << 24;
+constexpr int kTlGone = 0x60000000;  // above every ticket (tiles_fits)
 static_assert(sizeof(Diag64Smem) >= 2 * kTlStage * sizeof(float), "the stages take the engine's place");
 static_assert(sizeof(Diag64Smem) >= 2 * kTlB * kTlLd * sizeof(float), "P and T_j^T take the engine's place");
 
@@ -71,8 +75,7 @@ __device__ __forceinline__ bool t_above(int j, int N) { return ((N - 2 - j) & 1)
 // Rows m >= 32 of columns c < 32 are zero in every T^T, so that quarter of the
 // slot holds the counters instead (32 per row).
 constexpr int kTlSlot = kTlB * kTlB;
-constexpr int kTlTicket = 0;   // matrix 0 only: the next task
-constexpr int kTlAbort = 1;    // matrix 0 only: a wait gave up
+constexpr int kTlTicket = 0;   // matrix 0 only: the next task, or from kTlGone on: a wait gave up
 constexpr int kTlDone = 2;     // + j % 2: tiles below the diagonal finished in columns of that parity
 constexpr int kTlRow = 4;      // + i: tiles of row i finished so far
 constexpr int kTlMaxRows = 32 * 32 - kTlRow;
@@ -219,7 +222,7 @@ __device__ __forceinline__ void product(const float* A, const float* Bt, int ty,
 
 __global__ void __launch_bounds__(kTlThreads, kTlCtasPerSm)
     potrf_tiles_kernel(const float* __restrict__ a, float* l, int64_t batch, int n, int64_t group, int total,
-                       float* tws, int32_t* info) {
+                       float* tws, int32_t* info, uint32_t polls) {
   extern __shared__ __align__(16) unsigned char tl_raw[];
   float* const st0 = reinterpret_cast<float*>(tl_raw);  // two stages of (row tile, column tile)
   Diag64Smem& dg = *reinterpret_cast<Diag64Smem*>(tl_raw);
@@ -234,6 +237,7 @@ __global__ void __launch_bounds__(kTlThreads, kTlCtasPerSm)
     if (tid == 0) misc[0] = atomicAdd(tl_counter(tws, kTlTicket), 1);
     __syncthreads();
     const int ticket = misc[0];
+    if (ticket >= kTlGone) break;
     if (ticket >= total) return;
     // Ticket -> (group of matrices, tile in column order, matrix of the group).
     const int64_t g0 = (int64_t)ticket / (group * per) * group;
@@ -291,7 +295,7 @@ __global__ void __launch_bounds__(kTlThreads, kTlCtasPerSm)
     auto panels_ready = [&](int need) -> int {
       if (tid == 0) {
         int got = -1;
-        for (uint32_t p = 0; p < kTlPolls; ++p) {
+        for (uint32_t p = 0; p < polls; ++p) {
           const int pi = ld_relaxed(tl_counter(slot, kTlRow + i));
           const int pj = ld_relaxed(tl_counter(slot, diag ? kTlDone + (j & 1) : kTlRow + j));
           const int both = diag ? pi : min(pi, pj);
@@ -301,7 +305,7 @@ __global__ void __launch_bounds__(kTlThreads, kTlCtasPerSm)
             if (diag) misc[4] = pj == done_want;
             break;
           }
-          if ((p & 255) == 255 && ld_acquire(tl_counter(tws, kTlAbort)) != 0) break;
+          if ((p & 255) == 255 && ld_acquire(tl_counter(tws, kTlTicket)) >= kTlGone) break;
         }
         misc[1] = got;
       }
@@ -390,12 +394,12 @@ __global__ void __launch_bounds__(kTlThreads, kTlCtasPerSm)
       if (wait && !column_free) {
         if (tid == 0) {
           int got = 0;
-          for (uint32_t p = 0; p < kTlPolls; ++p) {
+          for (uint32_t p = 0; p < polls; ++p) {
             if (ld_acquire(tl_counter(slot, kTlDone + (j & 1))) == done_want) {
               got = 1;
               break;
             }
-            if ((p & 255) == 255 && ld_acquire(tl_counter(tws, kTlAbort)) != 0) break;
+            if ((p & 255) == 255 && ld_acquire(tl_counter(tws, kTlTicket)) >= kTlGone) break;
           }
           misc[1] = got;
         }
@@ -459,12 +463,12 @@ __global__ void __launch_bounds__(kTlThreads, kTlCtasPerSm)
         *reinterpret_cast<float4*>(P + (ty + 8 * r) * kTlLd + 4 * tx) = make_float4(c[r][0], c[r][1], c[r][2], c[r][3]);
       if (tid == 0) {
         int got = 0;
-        for (uint32_t p = 0; p < kTlPolls; ++p) {
+        for (uint32_t p = 0; p < polls; ++p) {
           if (ld_acquire(tl_counter(slot, kTlRow + j)) > j) {
             got = 1;
             break;
           }
-          if ((p & 255) == 255 && ld_acquire(tl_counter(tws, kTlAbort)) != 0) break;
+          if ((p & 255) == 255 && ld_acquire(tl_counter(tws, kTlTicket)) >= kTlGone) break;
         }
         misc[1] = got;
       }
@@ -514,11 +518,15 @@ __global__ void __launch_bounds__(kTlThreads, kTlCtasPerSm)
     __syncthreads();
     if (!ok) {
       // A wait gave up: nothing after it can be trusted.
-      if (tid == 0) atomicExch(tl_counter(tws, kTlAbort), 1);
-      if (info != nullptr)
-        for (int64_t q = tid; q < batch; q += kTlThreads) info[q] = -1;
-      return;
+      if (tid == 0) {
+        atomicExch(tl_counter(tws, kTlTicket), kTlGone);
+        __threadfence();
+      }
+      __syncthreads();
+      break;
     }
+    // L_jj and info come before this CTA's next ticket (see the end).
+    if (diag && tid == 0) __threadfence();
     if (!diag && tid == 0) {
       __threadfence();
       atomicExch(tl_counter(slot, kTlRow + i), j + 1);
@@ -526,6 +534,17 @@ __global__ void __launch_bounds__(kTlThreads, kTlCtasPerSm)
     }
     // The upper tile (j, i), unless T_j^T is there.
     if (!diag && !(i == j + 1 && t_above(j, N))) clear_tile(L, n, col0, row0);
+  }
+  // A wait gave up, here or elsewhere: mark the output.  Every store to a marked
+  // place is followed by a mark: each CTA draws a ticket after its own stores, and
+  // either that is past kTlGone and it marks them itself, or the marks of the CTA
+  // that gave up come after its draw and so after them.
+  if (info != nullptr)
+    for (int64_t q = tid; q < batch; q += kTlThreads) info[q] = -1;
+  const int64_t rows = batch * n;
+  for (int64_t q = tid; q < rows; q += kTlThreads) {
+    const int64_t b = q / n, r = q - b * n;
+    l[(size_t)b * n * n + (size_t)r * (n + 1)] = __int_as_float(0x7fc00000);
   }
 }
 
@@ -535,7 +554,11 @@ bool tiles_fits(int64_t batch, int64_t n) {
   return N <= kTlMaxRows && batch * (N * (N + 1) / 2) < (int64_t)1 << 30;
 }
 
-int potrf_tiles(const float* a, float* l, int64_t batch, int n, float* tws, int32_t* info, cudaStream_t s) {
+// `polls` bounds every wait.  stall (the diagnostic; -1: none): the matrix
+// whose finished tiles of the even columns are never counted to the number
+// that its diagonal tiles wait for.
+static int launch_tiles(const float* a, float* l, int64_t batch, int n, float* tws, int32_t* info, uint32_t polls,
+                        int64_t stall, cudaStream_t s) {
   const int N = (n + kTlB - 1) / kTlB;
   const int64_t total = batch * ((int64_t)N * (N + 1) / 2);
   const int64_t slots = (int64_t)device_sms() * kTlCtasPerSm;
@@ -550,12 +573,39 @@ int potrf_tiles(const float* a, float* l, int64_t batch, int n, float* tws, int3
   const cudaError_t e = cudaMemset2DAsync(tws + 32 * kTlB, kTlSlot * sizeof(float), 0, zero_rows * kTlB * sizeof(float),
                                           (size_t)batch, s);
   if (e != cudaSuccess) return set_error(B2P_ERR_CUDA, "cudaMemset2DAsync(counters): %s", cudaGetErrorString(e));
+  if (stall >= 0) {
+    // kTlDone + 0 starts far below zero.
+    const cudaError_t e2 = cudaMemsetAsync(tws + stall * kTlSlot + 32 * kTlB + kTlDone, 0x80, sizeof(int), s);
+    if (e2 != cudaSuccess) return set_error(B2P_ERR_CUDA, "cudaMemsetAsync(counter): %s", cudaGetErrorString(e2));
+  }
   {
     TraceScope ts(kKTiles, s, (double)batch * n * n * n / 3.0);
     potrf_tiles_kernel<<<(int)std::min<int64_t>(total, slots), kTlThreads, kTlSmem, s>>>(
-        a, l, batch, n, std::min<int64_t>(group, batch), (int)total, tws, info);
+        a, l, batch, n, std::min<int64_t>(group, batch), (int)total, tws, info, polls);
   }
   return check_launch("potrf_tiles_kernel");
 }
 
+int potrf_tiles(const float* a, float* l, int64_t batch, int n, float* tws, int32_t* info, cudaStream_t s) {
+  return launch_tiles(a, l, batch, n, tws, info, kTlPolls, -1, s);
+}
+
 }  // namespace b2p
+
+using namespace b2p;
+
+extern "C" int b2p_debug_potrf_tiles_stall(const float* a, float* l, int64_t batch, int64_t n, int64_t matrix,
+                                           uint32_t polls, void* workspace, size_t workspace_bytes, int32_t* info,
+                                           void* stream) {
+  set_error(B2P_OK, "%s", "");
+  if (a == nullptr || l == nullptr || a == l || batch <= 0 || n <= 128 || n > (1 << 20) || !tiles_fits(batch, n) ||
+      matrix < 0 || matrix >= batch || polls == 0 || polls > kTlPolls)
+    return set_error(B2P_ERR_INVALID_ARG, "bad arguments to b2p_debug_potrf_tiles_stall");
+  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(l) | reinterpret_cast<uintptr_t>(workspace)) & 15u)
+    return set_error(B2P_ERR_INVALID_ARG, "buffers must be 16-byte aligned");
+  const size_t need = blocked_workspace_bytes(batch, n, B2P_MODE_FP32);
+  if (workspace == nullptr || workspace_bytes < need)
+    return set_error(B2P_ERR_WORKSPACE, "workspace of %zu bytes required, %zu given", need, workspace_bytes);
+  return launch_tiles(a, l, batch, (int)n, static_cast<float*>(workspace), info, polls, matrix,
+                      static_cast<cudaStream_t>(stream));
+}

@@ -100,8 +100,10 @@ B2P_API size_t b2p_potrf_workspace_size(int64_t batch, int64_t n, int mode);
  *   info       optional device int32[batch]: 0 on success, k+1 when the
  *              k-th pivot was not positive (cuSOLVER potrf convention).  A
  *              non-SPD matrix yields NaN from the failing column on.  -1
- *              marks a matrix whose tensor-core update gave up a bounded
- *              device-side wait (its output is then incomplete).
+ *              marks a matrix whose factorization gave up a bounded
+ *              device-side wait (its output is then incomplete).  In FP32
+ *              mode a wait that gives up marks the whole batch, and the
+ *              diagonals of L are NaN then, with or without info.
  *   stream     cudaStream_t (as void*).
  */
 B2P_API int b2p_potrf_batched(const float* a, float* l, int64_t batch, int64_t n, int mode,
@@ -327,6 +329,19 @@ B2P_API int b2p_debug_tc_gemm(const float* a, const float* b, float* d, int64_t 
  */
 B2P_API int b2p_debug_tc_gemm_stall(const float* a, const float* b, float* d, int64_t count, int mode,
                                     uint32_t stall_polls, int32_t* err, void* stream);
+
+/*
+ * Diagnostic of the FP32 kernel's bounded waits (n > 128): b2p_potrf_batched
+ * in FP32 mode, except that every wait is bounded by `polls` (at most 2^24)
+ * and that matrix number `matrix` never counts its finished tiles to what its
+ * third diagonal tile waits for.  That wait runs out, every CTA leaves, info
+ * is -1 and the diagonal of L NaN for the whole batch, and the context stays
+ * usable.  workspace: b2p_potrf_workspace_size(batch, n, B2P_MODE_FP32) bytes.
+ * No counterpart in the reference.
+ */
+B2P_API int b2p_debug_potrf_tiles_stall(const float* a, float* l, int64_t batch, int64_t n, int64_t matrix,
+                                        uint32_t polls, void* workspace, size_t workspace_bytes, int32_t* info,
+                                        void* stream);
 
 /*
  * Launch trace: when enabled, every kernel the library launches is bracketed
