@@ -449,7 +449,9 @@ size_t blocked_workspace_bytes(int64_t batch, int64_t n, int mode) {
 namespace {
 // Per device: the stream the FP32 look-ahead runs the bulk of each trailing
 // update on, with the events that fork it from and join it to the caller's.
+// A call holds `busy` while it enqueues (the events are shared).
 struct TrailStream {
+  std::mutex busy;
   cudaStream_t stream = nullptr;
   cudaEvent_t fork = nullptr;
   cudaEvent_t join = nullptr;
@@ -535,9 +537,11 @@ int potrf_blocked(const float* a, float* l, int64_t batch, int n, int mode, void
   // FP32 look-ahead: diag, panel and the next column's update carry the
   // critical path, so they launch at the device's greatest priority.
   const int* prio = nullptr;
+  std::unique_lock<std::mutex> enqueuing;
   if (!tensor && n > kNB) {
     TrailStream* ts0 = nullptr;
     if (int st = trail_stream(&ts0)) return st;
+    enqueuing = std::unique_lock<std::mutex>(ts0->busy);
     prio = &ts0->priority;
   }
   for (int K0 = 0; K0 < n; K0 += outer) {

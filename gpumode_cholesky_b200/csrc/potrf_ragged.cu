@@ -142,8 +142,10 @@ constexpr int kRaggedMaxStreams = 8;
 
 namespace {
 // Per device: the library streams dense groups run on, with the events that
-// fork them from and join them to the caller's stream.
+// fork them from and join them to the caller's stream.  A call holds `busy`
+// while it enqueues (the events are shared).
 struct GroupStreams {
+  std::mutex busy;
   cudaStream_t st[kRaggedMaxStreams] = {};
   cudaEvent_t fork = nullptr;
   cudaEvent_t join[kRaggedMaxStreams] = {};
@@ -482,8 +484,10 @@ int b2p_potrf_ragged(const b2p_ragged_plan* plan, const void* tables, const floa
     auto check = [](cudaError_t e, const char* what) -> int {
       return e == cudaSuccess ? B2P_OK : set_error(B2P_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
     };
+    std::unique_lock<std::mutex> enqueuing;
     if (p.nstreams > 1) {
       if (int st = group_streams(&gs)) return st;
+      enqueuing = std::unique_lock<std::mutex>(gs->busy);
       if (int st = check(cudaEventRecord(gs->fork, s), "cudaEventRecord")) return st;
       for (int i = 1; i < p.nstreams; ++i)
         if (int st = check(cudaStreamWaitEvent(gs->st[i], gs->fork, 0), "cudaStreamWaitEvent")) return st;

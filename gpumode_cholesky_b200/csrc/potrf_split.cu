@@ -787,8 +787,11 @@ size_t split_workspace_bytes(int64_t batch, int64_t n) {
 
 namespace {
 // Per device: a second stream for the look-ahead part of the updates and
-// the events that fork it from and join it to the caller's stream.
+// the events that fork it from and join it to the caller's stream.  A call
+// holds `busy` while it enqueues: a wait takes the event's latest record, which
+// must be this call's own, not that of another host thread's call.
 struct SideStream {
+  std::mutex busy;
   cudaStream_t stream = nullptr;
   cudaEvent_t fork = nullptr;
   cudaEvent_t join[2] = {nullptr, nullptr};
@@ -856,6 +859,7 @@ int potrf_split(const float* a, float* l, int64_t batch, int n, int mode, void* 
     return set_error(B2P_ERR_WORKSPACE, "workspace of %zu bytes required, %zu given", need, ws_bytes);
   SideStream* side = nullptr;
   if (int st = side_stream(&side)) return st;
+  std::lock_guard<std::mutex> enqueuing(side->busy);
   uint8_t* copies = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ws) + 1023) & ~(uintptr_t)1023);
   float* pb[2];
   pb[0] = reinterpret_cast<float*>(copies + (size_t)batch * 2 * panel_copy_region_bytes(n));
