@@ -88,14 +88,36 @@ __device__ __forceinline__ void store_row16(float* dst, const float (&x)[16]) {
     reinterpret_cast<float4*>(dst)[c4] = make_float4(x[4 * c4], x[4 * c4 + 1], x[4 * c4 + 2], x[4 * c4 + 3]);
 }
 
+// How an update subtracts a panel's 16 products: product by product, or in sums
+// (the small orders), of all 16 or, for the matrix's first panel, of 2, 2, 4 and
+// 8 (FIRST_SUM_ENDS: the last of each, as a mask).  A sum costs one rounding at
+// the element's own size, and one at the sum's size per product.  On smooth
+// covariances the first few products take nearly all of an element away, and
+// what is rounded at the size of their sum is large against what remains; on
+// Gram matrices the element keeps its size, and every subtraction costs.  Error
+// of L against 64 bits, in units of the product-by-product 32-wide blocks with sums of 32
+// that this replaced, over orders 33 to 128 and four kinds of input (Gram
+// matrices, squared-exponential covariances in the unit cube, two shifts each,
+// a model of the roundings on the CPU): at most 1.00 (16 at a time throughout
+// up to 1.36, product by product up to 1.71, 4 at a time up to 1.08).
+enum Sums { kByProduct = 0, kSum16 = 1, kSumFirst = 2 };
+constexpr uint32_t kFirstSumEnds = 1u << 1 | 1u << 3 | 1u << 7 | 1u << 15;
+
 // The rank-16 update in register tiles of R rows by 4 columns, x[4r + c] -=
 // sum_m a_rm lt[m][c0 + c], m = 0..15 ascending.  The columns' factors come
 // from the L^T view, where a warp's reads of one m are contiguous; so do the
 // rows' (a_rm = rows[m][r]) or they are rows of S or T^T (TROWS, a_rm =
-// rows[r][m]).  SUM: x += instead, in packed pairs.
-template <int R, bool TROWS, bool SUM>
+// rows[r][m]).  Sums run in packed pairs.
+template <int R, bool TROWS, int SUMS>
 __device__ __forceinline__ void update_tile16(float (&x)[4 * R], const float* rows, const float* lt_c) {
-#pragma unroll 2
+  constexpr bool SUM = SUMS != kByProduct;
+  constexpr uint32_t kEnds = SUMS == kSumFirst ? kFirstSumEnds : 1u << 15;
+  float d[SUM ? 4 * R : 1];
+  if (SUM) {
+#pragma unroll
+    for (int q = 0; q < 4 * R; ++q) d[q] = 0.0f;
+  }
+#pragma unroll (SUMS == kSumFirst ? 4 : 2)
   for (int m = 0; m < 16; m += 4) {
     float a[4][R];
     if (TROWS) {
@@ -122,13 +144,20 @@ __device__ __forceinline__ void update_tile16(float (&x)[4 * R], const float* ro
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         if (SUM) {
-          fma2(x[4 * r + 0], x[4 * r + 1], a[p][r], b.x, b.y);
-          fma2(x[4 * r + 2], x[4 * r + 3], a[p][r], b.z, b.w);
+          fma2(d[4 * r + 0], d[4 * r + 1], a[p][r], b.x, b.y);
+          fma2(d[4 * r + 2], d[4 * r + 3], a[p][r], b.z, b.w);
         } else {
           x[4 * r + 0] = fmaf(-a[p][r], b.x, x[4 * r + 0]);
           x[4 * r + 1] = fmaf(-a[p][r], b.y, x[4 * r + 1]);
           x[4 * r + 2] = fmaf(-a[p][r], b.z, x[4 * r + 2]);
           x[4 * r + 3] = fmaf(-a[p][r], b.w, x[4 * r + 3]);
+        }
+      }
+      if (SUM && (SUMS == kSumFirst || p == 3) && (kEnds >> (m + p) & 1u) != 0) {
+#pragma unroll
+        for (int q = 0; q < 4 * R; ++q) {
+          x[q] -= d[q];
+          d[q] = 0.0f;
         }
       }
     }
@@ -137,9 +166,10 @@ __device__ __forceinline__ void update_tile16(float (&x)[4 * R], const float* ro
 
 // The tile's R rows of four at `dst` (row stride kD64Ld), less panels
 // k0 .. k1 - 1 of L (`rows`, `lt_c` as above, at panel 0): product by product,
-// or with SUM each panel's sum at once.
+// or with SUM in sums (`first`: panel 0 is the matrix's first).
 template <int R, bool TROWS, bool SUM = false>
-__device__ __forceinline__ void update_blocks(float* dst, const float* rows, const float* lt_c, int k0, int k1) {
+__device__ __forceinline__ void update_blocks(float* dst, const float* rows, const float* lt_c, int k0, int k1,
+                                              bool first = false) {
   float x[4 * R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -149,16 +179,12 @@ __device__ __forceinline__ void update_blocks(float* dst, const float* rows, con
 #pragma unroll 1
   for (int k = k0; k < k1; ++k) {
     const float* rk = rows + 16 * k * (TROWS ? 1 : kD64Ld);
-    if (SUM) {
-      float d[4 * R];
-#pragma unroll
-      for (int q = 0; q < 4 * R; ++q) d[q] = 0.0f;
-      update_tile16<R, TROWS, true>(d, rk, lt_c + 16 * k * kD64Ld);
-#pragma unroll
-      for (int q = 0; q < 4 * R; ++q) x[q] -= d[q];
-    } else {
-      update_tile16<R, TROWS, false>(x, rk, lt_c + 16 * k * kD64Ld);
-    }
+    if (!SUM)
+      update_tile16<R, TROWS, kByProduct>(x, rk, lt_c + 16 * k * kD64Ld);
+    else if (first && k == 0)
+      update_tile16<R, TROWS, kSumFirst>(x, rk, lt_c);
+    else
+      update_tile16<R, TROWS, kSum16>(x, rk, lt_c + 16 * k * kD64Ld);
   }
 #pragma unroll
   for (int r = 0; r < R; ++r)
@@ -287,12 +313,12 @@ __device__ __forceinline__ void t21_product(float* TT) {
 // inverse.  np < 4 leaves out panels that are identity padding.  BELOW: S has
 // 64 more rows (64 .. 127), which warps 4..7 solve along with the panels, 16
 // rows each; their updates are left-looking, since these warps never run out
-// of panel rows.  SUM: updates subtract a panel's sum at once, which rounds
-// less often at the element's own size (the small orders' form; the n > 128
-// paths keep the product-by-product order).
+// of panel rows.  SUM: updates subtract sums of products (Sums; the small
+// orders' form, `first` telling the matrix's first block; the n > 128 paths
+// keep the product-by-product order).
 template <bool INVERT, bool BELOW, bool SUM, class Bar>
-__device__ __forceinline__ void diag64_panels(float* S, float* Lt, float* TT, float* invd, int* bad, int np,
-                                              Bar bar) {
+__device__ __forceinline__ void diag64_panels(float* S, float* Lt, float* TT, float* invd, int* bad, int np, Bar bar,
+                                              bool first = false) {
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
@@ -306,9 +332,9 @@ __device__ __forceinline__ void diag64_panels(float* S, float* Lt, float* TT, fl
       const int r = 16 * ph + 2 * (tid >> 2), c = 16 * ph + 4 * (tid & 3);
       if (BELOW && tid >= kD64Threads) {
         const int rb = 2 * (tid >> 2);  // 64 ..
-        update_blocks<2, true, SUM>(S + rb * kD64Ld + c, S + rb * kD64Ld, Lt + c, 0, ph);
+        update_blocks<2, true, SUM>(S + rb * kD64Ld + c, S + rb * kD64Ld, Lt + c, 0, ph, first);
       } else if (r < 64) {
-        update_blocks<2, false, SUM>(S + r * kD64Ld + c, Lt + r, Lt + c, ph - 1, ph);
+        update_blocks<2, false, SUM>(S + r * kD64Ld + c, Lt + r, Lt + c, ph - 1, ph, first);
       }
       bar();
     }
@@ -346,7 +372,7 @@ __device__ __forceinline__ void diag64_panels(float* S, float* Lt, float* TT, fl
       // Panels before ph applied to the columns beyond block ph: warp 2 one
       // block ahead; two blocks ahead it is warp 3's where that has no T.
       const int q = 32 + (lane & ~3), i = ph + (warp == 2 ? 1 : 2), c = 16 * i + 4 * (lane & 3);
-      update_blocks<4, false, SUM>(S + q * kD64Ld + c, Lt + q, Lt + c, INVERT ? 0 : ph - 1, ph);
+      update_blocks<4, false, SUM>(S + q * kD64Ld + c, Lt + q, Lt + c, INVERT ? 0 : ph - 1, ph, first);
     } else if (INVERT && warp > 0 && warp < 4 && ph > 0) {
       // T, a row of T^T per column: warp 3 has columns 0..15, warp 1 16..31,
       // warp 2 32..63 (f: the first block row that is not zero).  Block row

@@ -124,8 +124,8 @@ __global__ void __launch_bounds__(kWarp32Warps * 32, 7)
 // 64 need the first block alone, on four warps.  Latency bounds it: one chain
 // of n pivots.  Measured on B200, us per call in a graph, against warp
 // factorizations of 32-wide blocks with a row solve and a 4x4-tile update
-// between them: 16x64 14.7 -> 6.6, 16x100 31.4 -> 15.2, 256x128 39.7 -> 23.2,
-// 2000x64 99.5 -> 34.7, 8000x48 392 -> 102, 3000x100 382 -> 212.
+// between them: 16x64 14.7 -> 6.9, 16x100 31.4 -> 15.5, 256x128 39.7 -> 23.6,
+// 2000x64 99.5 -> 35.0, 8000x48 392 -> 102, 3000x100 382 -> 215.
 template <bool BIG>
 constexpr int kCtaThreads = BIG ? 256 : kD64Threads;
 template <bool BIG>
@@ -143,16 +143,29 @@ __device__ __forceinline__ void cp_async(float* dst, const float* src, int bytes
 
 // S2[i][j] -= sum_m L21[i][m] L21[j][m] for j <= i < 64, m < 64; thread (ti, tj)
 // has rows ti + 16 r and columns tj + 16 c (neighbouring threads, neighbouring
-// rows: no bank conflicts), of which only r >= c matter.
+// rows: no bank conflicts), of which only r >= c matter.  A panel's products in
+// sums as in the block's own updates (Sums).
 __device__ __forceinline__ void lower_update64(float* S2, const float* L21) {
   const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
-  float acc[4][4];
+  float x[4][4], acc[4][4];
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) acc[r][c] = 0.0f;
-#pragma unroll 2
-  for (int m = 0; m < 64; m += 4) {
+    for (int c = 0; c <= r; ++c) {
+      x[r][c] = S2[(ti + 16 * r) * kD64Ld + tj + 16 * c];
+      acc[r][c] = 0.0f;
+    }
+  auto subtract = [&] {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c <= r; ++c) {
+        x[r][c] -= acc[r][c];
+        acc[r][c] = 0.0f;
+      }
+  };
+  // Columns m .. m + 3; `ends` as kFirstSumEnds, for these four.
+  auto products = [&](int m, uint32_t ends) {
     float a[4][4], b[4][4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
@@ -162,16 +175,26 @@ __device__ __forceinline__ void lower_update64(float* S2, const float* L21) {
       b[r][0] = u.x, b[r][1] = u.y, b[r][2] = u.z, b[r][3] = u.w;
     }
 #pragma unroll
-    for (int p = 0; p < 4; ++p)
+    for (int p = 0; p < 4; ++p) {
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
         for (int c = 0; c <= r; ++c) acc[r][c] = fmaf(a[r][p], b[c][p], acc[r][c]);
+      if ((ends >> p & 1u) != 0) subtract();
+    }
+  };
+#pragma unroll
+  for (int m = 0; m < 16; m += 4) products(m, kFirstSumEnds >> m & 15u);
+#pragma unroll 1
+  for (int g = 16; g < 64; g += 16) {
+#pragma unroll 2
+    for (int m = 0; m < 16; m += 4) products(g + m, 0u);
+    subtract();
   }
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int c = 0; c <= r; ++c) S2[(ti + 16 * r) * kD64Ld + tj + 16 * c] -= acc[r][c];
+    for (int c = 0; c <= r; ++c) S2[(ti + 16 * r) * kD64Ld + tj + 16 * c] = x[r][c];
 }
 
 template <bool BIG>
@@ -216,7 +239,7 @@ __global__ void __launch_bounds__(kCtaThreads<BIG>, BIG ? 2 : 4)
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    diag64_panels<false, BIG, true>(S1, Lt, nullptr, invd, bad, pad == 64 ? (n + 15) / 16 : 4, CtaBarrier());
+    diag64_panels<false, BIG, true>(S1, Lt, nullptr, invd, bad, pad == 64 ? (n + 15) / 16 : 4, CtaBarrier(), true);
     if (BIG && n > 64) {
       lower_update64(S2, S1 + 64 * kD64Ld);
       __syncthreads();
