@@ -461,7 +461,9 @@ __global__ void __launch_bounds__(kTrsvThreads, 2) trsv_kernel(const float* __re
 // whole lower triangle is copied to shared memory at once, and the loops stay
 // loops.  Thread i has row i of L (column i for L^T); warp k solves diagonal
 // block k with one shuffle per pivot, and the others subtract its 32 solved
-// values.  Same values as above for L; L^T sums a block's 32 products in order.
+// values.  Same values as above (for L^T those of n % 4 == 0: a block's 32
+// products in eight sums of four, added in pairs; in one sum x was up to 1.3 times
+// further off, on covariances of order 128).
 // Device us before and now: 256x128 GP forward 31 -> 12, solve with L^T and
 // Lbar 42 -> 19 (one launch of two); per call in a graph 16x100 28 -> 10 and
 // 27 -> 16, 8x33 16.7 -> 7.1.
@@ -522,8 +524,23 @@ __global__ void __launch_bounds__(kSmallMaxN) trsv_small_kernel(const float* __r
       if (TRANS ? i < r0 : (i >= r0 + 32 && i < n)) {
         float acc = 0.0f;
         if (TRANS) {
-#pragma unroll 8
-          for (int j = 0; j < w; ++j) acc = fmaf(ss[(r0 + j) * ld + i], xs[r0 + j], acc);
+          // Eight sums of four, added in pairs.  Only the last block, the first
+          // here, is ever partial.
+          auto sum4 = [&](int j0, int j1) {
+            float p = 0.0f;
+#pragma unroll
+            for (int j = j0; j < j0 + 4; ++j)
+              p = fmaf(j < j1 ? ss[(r0 + j) * ld + i] : 0.0f, xs[r0 + j], p);
+            return p;
+          };
+          if (w == 32) {
+#pragma unroll 2
+            for (int j = 0; j < 32; j += 16)
+              acc += (sum4(j, 32) + sum4(j + 4, 32)) + (sum4(j + 8, 32) + sum4(j + 12, 32));
+          } else {
+#pragma unroll 1
+            for (int j = 0; j < w; j += 16) acc += (sum4(j, w) + sum4(j + 4, w)) + (sum4(j + 8, w) + sum4(j + 12, w));
+          }
         } else {
 #pragma unroll 2
           for (int j = 0; j < 32; j += 4) {

@@ -15,6 +15,7 @@ import pytest
 import torch
 
 from gpumode_cholesky_b200 import cholesky
+from gpumode_cholesky_b200.gp import trsv
 
 pytestmark = pytest.mark.gpu
 
@@ -76,3 +77,29 @@ def test_factor_no_further_off_than_blocks_of_32(n, kind):
     exact = np.linalg.cholesky(a.astype(np.float64))
     got = cholesky(torch.from_numpy(a).cuda(), mode="fp32").cpu().numpy()
     assert _rms(got, exact) <= SLACK * _rms(_factor_blocks_of_32(a), exact)
+
+
+def _solve_transposed(l: np.ndarray, b: np.ndarray) -> np.ndarray:
+    """L^T x = b in blocks of 32 rows: a block's products in eight sums of four, added in pairs."""
+    x, n = b.copy(), b.shape[1]
+    inv = np.float32(1.0) / l[:, range(n), range(n)]
+    for r0 in range((n - 1) // 32 * 32, -1, -32):
+        e = min(n, r0 + 32)
+        for j in range(e - 1, r0 - 1, -1):
+            x[:, j] *= inv[:, j]
+            x[:, r0:j] = _fma(-l[:, j, r0:j], x[:, j : j + 1], x[:, r0:j])
+        p = np.zeros((8, x.shape[0], r0), dtype=np.float32)
+        for j in range(r0, e):
+            p[(j - r0) // 4] = _fma(l[:, j, :r0], x[:, j : j + 1], p[(j - r0) // 4])
+        x[:, :r0] -= ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]))
+    return x
+
+
+@pytest.mark.parametrize("n", [40, 64, 67, 96, 128])
+@pytest.mark.parametrize("noise", [0.1, 0.001])
+def test_transposed_solve_no_further_off_than_sums_of_four(n, noise):
+    l = np.linalg.cholesky(_covariances(n, noise, n + 1).astype(np.float64)).astype(np.float32)
+    b = np.random.default_rng(n).standard_normal((BATCH, n)).astype(np.float32)
+    exact = np.linalg.solve(l.astype(np.float64).transpose(0, 2, 1), b.astype(np.float64)[..., None])[..., 0]
+    got = trsv(torch.from_numpy(l).cuda(), torch.from_numpy(b).cuda(), trans=True).cpu().numpy()
+    assert _rms(got, exact) <= SLACK * _rms(_solve_transposed(l, b), exact)
