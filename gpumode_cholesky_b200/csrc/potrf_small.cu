@@ -66,29 +66,20 @@ __global__ void __launch_bounds__(kWarp32Warps * 32, 7)
     }
     __syncwarp();
     float x[32];
-    auto load_row = [&] {
 #pragma unroll
-      for (int c4 = 0; c4 < 8; ++c4) {
-        const float4 v = *reinterpret_cast<const float4*>(t + lane * kStageLd + 4 * c4);
-        x[4 * c4 + 0] = v.x;
-        x[4 * c4 + 1] = v.y;
-        x[4 * c4 + 2] = v.z;
-        x[4 * c4 + 3] = v.w;
-      }
-      if (n < 32) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (lane >= n || j >= n) x[j] = (lane == j) ? 1.0f : 0.0f;
-      }
-    };
-    load_row();
-    int bad = warp_factor32<true>(x, lane, n, colbuf[warp]);
-    if (bad != 0) {
-      load_row();
-      bad = warp_factor32<false>(x, lane, n, colbuf[warp]);
-    } else {
-      bad = -1;
+    for (int c4 = 0; c4 < 8; ++c4) {
+      const float4 v = *reinterpret_cast<const float4*>(t + lane * kStageLd + 4 * c4);
+      x[4 * c4 + 0] = v.x;
+      x[4 * c4 + 1] = v.y;
+      x[4 * c4 + 2] = v.z;
+      x[4 * c4 + 3] = v.w;
     }
+    if (n < 32) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (lane >= n || j >= n) x[j] = (lane == j) ? 1.0f : 0.0f;
+    }
+    const int bad = warp_factor32(x, lane, n, colbuf[warp]);
     __syncwarp();
 #pragma unroll
     for (int c4 = 0; c4 < 8; ++c4) {

@@ -15,10 +15,8 @@ namespace b2p {
 
 // Factor the 32x32 block x[] (row `lane`), columns >= w / rows >= w are
 // identity padding.  On return x holds L (lower part valid, upper part is
-// don't-care).  NORMAL (see rsqrt_refined): returns 0, or a non-zero value if
-// a pivot was not a normal positive number, and the caller starts again with
-// the general form; that returns the first local pivot index that was not
-// positive, or -1.  All 32 lanes must call.
+// don't-care).  Returns the first local pivot index that was not positive, or
+// -1.  All 32 lanes must call.
 //
 // Step k takes the pivot d = x[k] of lane k and, in the same round of
 // shuffles, lane k+1's unscaled column-k value e; every lane then forms
@@ -29,9 +27,15 @@ namespace b2p {
 // instruction, right after shuffling out its own pivot, in the shadow of that
 // pivot's reciprocal square root.  The arithmetic is the same as the textbook
 // right-looking update, value for value and in the same order.
-template <bool NORMAL>
+//
+// One form for all pivots: the rsqrt that takes normal ones only saves 23 cycles
+// in each step, but a warp whose matrix has another pivot starts again, and the
+// two forms' code together cost more than that (us in a graph, two forms / this
+// one / before the packed pairs: 20000x32 48.8 / 46.0 / 48.3, 20000x1 21.2 / 18.7
+// / 20.0, 4096x32 12.2 / 12.1 / 12.5, 20000x24 53.4 / 54.3 / 58.7; every matrix
+// failing, 20000x32 83.7 / 46.0 / 48.3).
 __device__ __forceinline__ int warp_factor32(float (&x)[32], int lane, int w, float* colbuf) {
-  int bad = NORMAL ? 0 : -1;
+  int bad = -1;
   float nlprev = 0.0f;  // minus this lane's L[lane][k-1]
 #pragma unroll
   for (int k = 0; k < 32; ++k) {
@@ -55,11 +59,8 @@ __device__ __forceinline__ int warp_factor32(float (&x)[32], int lane, int w, fl
           }
         }
       }
-      if (NORMAL)
-        bad |= pivot_normal(d) ? 0 : 1;
-      else if (bad < 0 && pivot_bad(d))
-        bad = k;
-      const float y = rsqrt_refined<NORMAL>(d);
+      if (bad < 0 && pivot_bad(d)) bad = k;
+      const float y = rsqrt_refined(d);
       x[k] = (lane == k) ? d * y : x[k] * y;
       nlprev = -x[k];
       if (k + 1 < 32) x[k + 1] = fmaf(nlprev, e * y, x[k + 1]);
