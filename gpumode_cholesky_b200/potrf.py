@@ -58,7 +58,7 @@ def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     return buf
 
 
-@functools.lru_cache(maxsize=256)
+@functools.lru_cache(maxsize=256, typed=True)  # typed: 1.0 is no mode though it equals 1
 def resolve_mode(mode: str | int | None, n: int) -> int:
     """Precision mode code for order n; None picks the library default (FP32).
 
