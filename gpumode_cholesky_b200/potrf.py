@@ -21,10 +21,28 @@ from . import _lib
 _WS: dict[tuple[int, int], torch.Tensor] = {}
 _SAME_DEVICE = contextlib.nullcontext()
 
+
+class _BackTo:
+    """Makes a device current again on leaving, as ``torch.cuda.device`` does."""
+
+    __slots__ = ("index",)
+
+    def __init__(self, index: int):
+        self.index = index
+
+    def __enter__(self) -> None:
+        pass
+
+    def __exit__(self, *exc) -> bool:
+        torch._C._cuda_maybeExchangeDevice(self.index)
+        return False
+
+
 # The smallest calls are bound by the host (a 4096x32 call's kernel takes about
 # as long as enqueueing it), so a call looks up only what it needs: the raw
-# stream handle instead of a Stream object, no device switch when the device is
-# the current one, and sizes that depend on the shape alone from a small cache.
+# stream handle instead of a Stream object, no device to go back to when the
+# device is the current one, and sizes that depend on the shape alone from a small
+# cache.
 
 
 def _stream_ptr(device: torch.device) -> int:
@@ -34,8 +52,16 @@ def _stream_ptr(device: torch.device) -> int:
 
 
 def _on_device(device: torch.device):
-    """Context that makes `device` current, free of cost when it is already."""
-    return _SAME_DEVICE if torch._C._cuda_getDevice() == device.index else torch.cuda.device(device)
+    """Makes `device` current; the context returned goes back to the one before, if that is another.
+
+    By an exchange, as ``torch.cuda.device`` does it, and not by asking which
+    device is current: torch can answer with one that it has yet to switch to,
+    while the library's launches go where the CUDA runtime is.
+    """
+    if device.index is None:
+        return torch.cuda.device(device)
+    before = torch._C._cuda_exchangeDevice(device.index)
+    return _SAME_DEVICE if before == device.index else _BackTo(before)
 
 
 @functools.lru_cache(maxsize=256)
