@@ -758,12 +758,24 @@ __global__ void fp8_scale_kernel(const float* __restrict__ a, float* __restrict_
 // The width, in block columns, of the outer blocks that the older panels are
 // applied to at a time (split_wide_kernel), or 0 for none.  Without it every
 // column reads all earlier panels of 128 x 64 tiles, 48 KB per 2^19
-// multiply-adds, and from some 100 block rows of matrices on that outlasts the
-// step it hides behind (1 x 8192: the middle steps waited 6 us each).  Measured
-// on B200 with two step CTAs per SM, us, none / 4 / 8: 1x4096 1314 / 1367 /
-// 1335, 2x3072 1036 / 1046 / 1030, 1x6144 2151 / 2136 / 2123, 1x7168 2615 /
-// 2466 / 2482, 1x8192 3369 / 2858 / 2924, 1x10240 5424 / 3994 / 4007, 4x3072
-// 1163 / 1107 / 1152, 8x2048 812 / 761 / 804, 16x1536 717 / 685 / 724.
+// multiply-adds, which outlasts the step it hides behind once the matrices
+// together are large (1 x 8192: the middle steps waited 6 us each).  It also
+// rounds less: an outer block's sum leaves the tensor core's accumulator, which
+// does not round to nearest, every W panels.  Measured on B200 with two step CTAs
+// per SM, us, none / 4 wide (the calls where 4 is the slower side are kept on it
+// for their error, which TF32 and FP8 do not see):
+//   BF16x3  7x1088 350 / 358, 15x1152 405 / 419, 5x1536 511 /
+//           513, 8x2048 739 / 741, 7x2560 990 / 1013, 1x6720 2313 / 2322, 1x7168
+//           2459 / 2456, 1x8192 2837 / 2817, 13x2048 965 / 936, 60x1280 1038 / 973,
+//           3x5120 2167 / 1996, 2x7168 3251 / 2791, 1x10240 4276 / 3863; with more
+//           matrices than the steps' SMs, 80x1536 1885 / 2138, 160x1088 1643 / 2062
+//   TF32    5x1536 489 / 504, 4x2048 655 / 669, 1x8192 2750 / 2737, 3x5120 2093 /
+//           1902, 80x1536 1846 / 2086
+//   FP8     5x1536 511 / 529, 4x2048 663 / 693, 1x8192 2837 / 2866, 3x5120 2157 /
+//           1991, 1x10240 4240 / 3864, 80x1536 1917 / 2242
+// Error of L against 64 bits, BF16x3, G G^T / n + 0.1 I, none / 4: 7x1088 2.73e-6 /
+// 2.73e-6, 8x2048 3.17e-6 / 2.91e-6, 1x7040 3.75e-6 / 2.97e-6, 80x1536 4.20e-6 /
+// 2.94e-6.
 constexpr int kWideMinRows = 104;   // batch x block rows
 constexpr int kWideLargeN = 12288;  // 8 from here (1 x 16384: 8 best of 4, 8, 16)
 static_assert(64 * 4 % kXCols == 0, "outer blocks are whole wide tiles");
