@@ -776,12 +776,18 @@ __global__ void fp8_scale_kernel(const float* __restrict__ a, float* __restrict_
 // Error of L against 64 bits, BF16x3, G G^T / n + 0.1 I, none / 4: 7x1088 2.73e-6 /
 // 2.73e-6, 8x2048 3.17e-6 / 2.91e-6, 1x7040 3.75e-6 / 2.97e-6, 80x1536 4.20e-6 /
 // 2.94e-6.
+//
+// The two buffers take 2048 bytes a row, up to half of a small matrix: beyond 2
+// GiB together there are none, so that batches which fill the GPU's memory still
+// fit (13 500 x 1088: A, L and the rest of the workspace 165 GB, buffers 30 GB).
 constexpr int kWideMinRows = 104;   // batch x block rows
+constexpr int64_t kWideMaxBytes = (int64_t)2 << 30;
+constexpr int64_t kWideRowBytes = 2 * 4 * 64 * sizeof(float);
 constexpr int kWideLargeN = 12288;  // 8 from here (1 x 16384: 8 best of 4, 8, 16)
 static_assert(64 * 4 % kXCols == 0, "outer blocks are whole wide tiles");
 static int wide_width(int64_t batch, int64_t n) {
   if (n >= kWideLargeN) return 8;
-  return batch * (n / 64) >= kWideMinRows ? 4 : 0;
+  return batch * (n / 64) >= kWideMinRows && batch * n * kWideRowBytes <= kWideMaxBytes ? 4 : 0;
 }
 
 // Panel copies, then two per-matrix FP32 panel buffers (n x 64 each; block
@@ -794,7 +800,11 @@ static size_t split_sig_offset(int64_t batch, int64_t n) {
 }
 size_t split_workspace_bytes(int64_t batch, int64_t n) {
   // ... then the FP8 mode's block scales (batch x n/64 floats).
-  return split_sig_offset(batch, n) + (((size_t)batch * (n / 64) * sizeof(float) + 255) & ~(size_t)255) + 1024;
+  const size_t own = split_sig_offset(batch, n) + (((size_t)batch * (n / 64) * sizeof(float) + 255) & ~(size_t)255) + 1024;
+  // Never less than for a smaller batch: one workspace serves all up to its own.
+  const int64_t widest = kWideMaxBytes / (n * kWideRowBytes);
+  return n < kWideLargeN && batch > widest && wide_width(widest, n) > 0 ? std::max(own, split_workspace_bytes(widest, n))
+                                                                        : own;
 }
 
 namespace {
