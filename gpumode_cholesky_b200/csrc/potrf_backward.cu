@@ -226,8 +226,8 @@ __global__ void __launch_bounds__(Bs<NP>::kThreads)
         bB[i * kLd + j] = in ? G[(size_t)i * n + j] : 0.0f;
       }
     __syncthreads();
+    static_assert(Bs<NP>::kThreads >= NP, "a thread for each diagonal element");
     if (tid < NP) invd[tid] = 1.0f / bA[tid * kLd + tid];
-    if (Bs<NP>::kThreads < NP) __syncthreads();
     // P = Phi(L^T Lbar) (tiles reaching the lower triangle; k >= max(i, j)),
     // kept in registers.
     const bool lower = 4 * tj <= 8 * ti + 7;
