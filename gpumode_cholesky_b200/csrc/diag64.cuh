@@ -90,16 +90,16 @@ __device__ __forceinline__ void store_row16(float* dst, const float (&x)[16]) {
 
 // How an update subtracts a panel's 16 products: product by product, or in sums
 // (the small orders), of all 16 or, for the matrix's first panel, of 2, 2, 4 and
-// 8 (FIRST_SUM_ENDS: the last of each, as a mask).  A sum costs one rounding at
+// 8 (kFirstSumEnds: the last of each, as a mask).  A sum costs one rounding at
 // the element's own size, and one at the sum's size per product.  On smooth
 // covariances the first few products take nearly all of an element away, and
 // what is rounded at the size of their sum is large against what remains; on
 // Gram matrices the element keeps its size, and every subtraction costs.  Error
-// of L against 64 bits, in units of the product-by-product 32-wide blocks with sums of 32
-// that this replaced, over orders 33 to 128 and four kinds of input (Gram
-// matrices, squared-exponential covariances in the unit cube, two shifts each,
-// a model of the roundings on the CPU): at most 1.00 (16 at a time throughout
-// up to 1.36, product by product up to 1.71, 4 at a time up to 1.08).
+// of L against 64 bits over that of product-by-product 32-wide blocks with sums
+// of 32 between them, which this replaced, at orders 33 to 128 on Gram matrices
+// and squared-exponential covariances in the unit cube, two shifts each (a model
+// of the roundings on the CPU): 0.45 to 1.00; 16 at a time throughout up to
+// 1.36, product by product up to 1.71, 4 at a time up to 1.08.
 enum Sums { kByProduct = 0, kSum16 = 1, kSumFirst = 2 };
 constexpr uint32_t kFirstSumEnds = 1u << 1 | 1u << 3 | 1u << 7 | 1u << 15;
 

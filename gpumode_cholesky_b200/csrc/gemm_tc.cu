@@ -10,7 +10,7 @@
 // wanted, and apply Phi (keep the lower triangle, halve the diagonal) in the
 // epilogue.  One 256-thread CTA per output tile: per 64-wide K chunk every
 // thread stages one operand row (128B-swizzled K-major, BF16 hi/lo split or
-// TF32), thread 0 issues the MMAs into a 128x128 FP32 TMEM accumulator, and
+// TF32), an elected lane issues the MMAs into a 128x128 FP32 TMEM accumulator, and
 // the epilogue reads TMEM with tcgen05.ld.  Waits are bounded.
 //
 // A triangular hint also means that the other triangle is not read: elements

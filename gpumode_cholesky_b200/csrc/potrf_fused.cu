@@ -130,8 +130,9 @@ __global__ void __launch_bounds__(kFThreads, 2)
   umma::fence_after_sync();
   const uint32_t tmem = *tslot;
 
-  // mbarrier phase bookkeeping (thread 0 drives full/empty; all wait on done)
-  // Bit s: parity of stage s's next phase.
+  // Phases: all threads wait on done; full and empty are driven by warp 0's
+  // elected lane, the same one each time, and their bits (bit s: parity of stage
+  // s's next phase) are valid in that lane alone.
   uint32_t ph_full = 0u, ph_empty = 0u;
   uint32_t ph_done = 0u;
   bool ok = true;

@@ -8,7 +8,7 @@
 //      the 128B-swizzled K-major layout, converting on the way:
 //        TF32   : the value rounded to TF32 (cvt.rna), 2 swizzle atoms per row;
 //        BF16x3 : hi = bf16(x) and lo = bf16(x - hi) in two separate tiles;
-//   3. thread 0 issues the MMAs (TF32: 8 x K=8; BF16x3: 4 x K=16 for each of
+//   3. an elected lane issues the MMAs (TF32: 8 x K=8; BF16x3: 4 x K=16 for each of
 //      hi*hi, hi*lo, lo*hi) and commits them to an mbarrier;
 //   4. each warp reads its 32 accumulator rows from TMEM (tcgen05.ld) and
 //      writes C - D to L for the lower-triangular part.
