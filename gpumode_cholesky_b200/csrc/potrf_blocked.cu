@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(kD64Threads, 3)
       }
     }
     __syncthreads();
-    const int bad = diag64_factor_invert(sm);
+    int bad = diag64_factor_invert(sm);
+    if (bad >= w) bad = -1;  // padding behind a pivot that is infinite
     // L_kk (zeros above its diagonal; the engine leaves them in S).
     if (vec) {
 #pragma unroll

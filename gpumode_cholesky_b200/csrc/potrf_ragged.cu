@@ -108,7 +108,10 @@ __global__ void __launch_bounds__(kCopyThreads) ragged_scatter_kernel(const floa
   for (int64_t it = blockIdx.x; it < nitems; it += gridDim.x) {
     const int2 item = items[it];
     const DenseEntry e = ent[item.x];
-    if (item.y == 0 && threadIdx.x == 0 && info != nullptr) info[e.idx] = ginfo[item.x];
+    if (item.y == 0 && threadIdx.x == 0 && info != nullptr) {
+      const int32_t first = ginfo[item.x];
+      info[e.idx] = first <= e.n ? first : 0;  // beyond: padding behind a pivot that is infinite
+    }
     for (int rr = warp; rr < kCopyRows; rr += kCopyThreads / 32) {
       const int r = item.y + rr;
       if (r >= e.n) break;

@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kCtaThreads<BIG>, BIG ? 2 : 4)
       int first = 0;
       for (int p = 0; p < (BIG && n > 64 ? 8 : 4) && first == 0; ++p)
         if (bad[p] >= 0) first = 16 * p + bad[p] + 1;
-      info[mat] = first;
+      info[mat] = first <= n ? first : 0;  // beyond: padding behind a pivot that is infinite
     }
     __syncthreads();
   }

@@ -423,9 +423,10 @@ __global__ void __launch_bounds__(kTlThreads, kTlCtasPerSm)
         }
       }
       if (ok && info != nullptr && tid == 0) {
+        // Only the last tile has padding, and only a pivot that is infinite makes it bad.
         if (j == 0)
           info[b] = bad >= 0 ? bad + 1 : 0;
-        else if (bad >= 0 && __ldcg(info + b) == 0)
+        else if (bad >= 0 && col0 + bad < n && __ldcg(info + b) == 0)
           info[b] = col0 + bad + 1;
       }
       __syncthreads();
