@@ -130,12 +130,12 @@ struct TrsvShared {
   float part[2];       // this CTA's partial loss sums (GP)
 };
 
-// x (this CTA's rows, holding b on entry) <- L^{-1} x or L^{-T} x.
+// x (this CTA's rows, holding b on entry) <- L^{-1} x or L^{-T} x, for rows that
+// cannot be read as vectors (cluster_trsv_ahead has the others).
 template <bool TRANS>
 __device__ void cluster_trsv(const float* __restrict__ L, int n, float* x, TrsvShared& sh, int C, int rank) {
   const int tid = threadIdx.x;
   const int nb = (n + 31) / 32;
-  const bool vec = (n & 3) == 0;
   for (int s = 0; s < nb; ++s) {
     const int blk = TRANS ? nb - 1 - s : s;
     const int r0 = 32 * blk, m = min(32, n - r0);
@@ -170,8 +170,8 @@ __device__ void cluster_trsv(const float* __restrict__ L, int n, float* x, TrsvS
         const int i2 = 32 * (first + (idx2 >> 5) * C) + (idx2 & 31);
         const bool ok1 = i < n, ok2 = idx2 < rows && i2 < n;
         float a1 = 0.0f, a2 = 0.0f;
-        if (ok1) a1 = row_dot32(L + (size_t)i * n + r0, sh.xb, vec);
-        if (ok2) a2 = row_dot32(L + (size_t)i2 * n + r0, sh.xb, vec);
+        if (ok1) a1 = row_dot32(L + (size_t)i * n + r0, sh.xb, false);
+        if (ok2) a2 = row_dot32(L + (size_t)i2 * n + r0, sh.xb, false);
         if (ok1) x[i] -= a1;
         if (ok2) x[i2] -= a2;
       }
@@ -179,39 +179,19 @@ __device__ void cluster_trsv(const float* __restrict__ L, int n, float* x, TrsvS
       // own rows above the block: x[i] -= sum_j L[r0+j, i] xb[j] (column
       // reads, coalesced across threads)
       const int nown = blk > rank ? (blk - 1 - rank) / C + 1 : 0;
-      if (vec) {
-        for (int idx = tid; idx < 8 * nown; idx += kTrsvThreads) {
-          const int i = 32 * (rank + (idx >> 3) * C) + 4 * (idx & 7);
-          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int idx = tid; idx < 32 * nown; idx += kTrsvThreads) {
+        const int i = 32 * (rank + (idx >> 5) * C) + (idx & 31);
+        float acc = 0.0f;
 #pragma unroll 8
-          for (int j = 0; j < m; ++j) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(L + (size_t)(r0 + j) * n + i));
-            const float w = sh.xb[j];
-            acc.x = fmaf(v.x, w, acc.x);
-            acc.y = fmaf(v.y, w, acc.y);
-            acc.z = fmaf(v.z, w, acc.z);
-            acc.w = fmaf(v.w, w, acc.w);
-          }
-          x[i] -= acc.x;
-          x[i + 1] -= acc.y;
-          x[i + 2] -= acc.z;
-          x[i + 3] -= acc.w;
-        }
-      } else {
-        for (int idx = tid; idx < 32 * nown; idx += kTrsvThreads) {
-          const int i = 32 * (rank + (idx >> 5) * C) + (idx & 31);
-          float acc = 0.0f;
-#pragma unroll 8
-          for (int j = 0; j < m; ++j) acc = fmaf(__ldg(L + (size_t)(r0 + j) * n + i), sh.xb[j], acc);
-          x[i] -= acc;
-        }
+        for (int j = 0; j < m; ++j) acc = fmaf(__ldg(L + (size_t)(r0 + j) * n + i), sh.xb[j], acc);
+        x[i] -= acc;
       }
     }
     __syncthreads();
   }
 }
 
-// The same solve for n % 4 == 0 with the loads of L issued one step ahead:
+// The same solve for n % 4 == 0 and a 16-byte boundary, with the loads of L issued one step ahead:
 // the next step's diagonal block (by its owner's warp 0) while this step's
 // update runs, and this thread's first operands of the next update right
 // after this one, so that a step's critical path is the diagonal block's
@@ -410,7 +390,7 @@ __global__ void __launch_bounds__(kTrsvThreads, 2) trsv_kernel(const float* __re
       if (i < n) xs[i] = b[(size_t)m * n + i];
     }
     __syncthreads();
-    if ((n & 3) == 0)
+    if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(l) & 15u) == 0)
       cluster_trsv_ahead<TRANS>(L, n, xs, sh, C, rank);
     else
       cluster_trsv<TRANS>(L, n, xs, sh, C, rank);
@@ -608,7 +588,7 @@ int launch_small(const float* l, const float* b, float* x, float* loss, const fl
   return check_launch("trsv_small_kernel");
 }
 
-// Lbar, one warp per row (matrix, i); float4 stores when n % 4 == 0.
+// Lbar, one warp per row (matrix, i); float4 stores where its rows allow them.
 __global__ void __launch_bounds__(kTrsvThreads) gp_lbar_kernel(const float* __restrict__ l,
                                                                const float* __restrict__ alpha,
                                                                const float* __restrict__ beta,
@@ -630,7 +610,7 @@ __global__ void __launch_bounds__(kTrsvThreads) gp_lbar_kernel(const float* __re
       const float v = -bi * __ldg(a + j);
       return j == i ? v + dinv : v;
     };
-    if ((n & 3) == 0) {
+    if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(lbar) & 15u) == 0) {
       for (int j = 4 * lane; j < n; j += 128)
         *reinterpret_cast<float4*>(out + j) = make_float4(val(j), val(j + 1), val(j + 2), val(j + 3));
     } else {
